@@ -29,6 +29,7 @@ UNITS = {
     "refine.cu": [],
     "tridiag_dc.cu": [],
     "syevd2.cu": [],
+    "bulge.cu": [],
     "tc_mixed.cu": [],
     "tc_ozaki.cu": [],
     "chan_eig.cu": [],

@@ -15,7 +15,7 @@
 //      (one GEMM of inner size 2 NB over the [V | Y | V] buffer);
 //   2. band -> tridiagonal: bulge chasing (sweeps of Householder reflectors of
 //      length NB, each annihilating one column and chasing the bulge down the
-//      band), one persistent cooperative kernel (syevd2 stage 2 below);
+//      band), one persistent cooperative kernel (bulge.cu);
 //   3. tridiagonal eigenpairs by divide and conquer (tridiag_dc.cu);
 //   4. back-transformation: the stage-2 reflectors (in blocks of NB sweeps) and
 //      the stage-1 panels (compact WY, GEMMs), applied to the eigenvectors.
@@ -27,22 +27,13 @@
 
 #include "ctx.h"
 #include "dgemm.h"
+#include "syevd2.h"
 
 namespace bsrg {
 namespace {
 
-constexpr int NB = 32;              // bandwidth of the intermediate band matrix
 constexpr int PQ_ROWS = 512;        // panel rows held in shared memory per CTA
 constexpr int PQ_NT = 256;
-constexpr unsigned long long WAIT_NS = 2000000000ull;   // bound of every device-side wait (2 s)
-
-__device__ __forceinline__ unsigned long long gtime()
-{
-    unsigned long long t;
-    asm volatile("mov.u64 %0, %%globaltimer;" : "=l"(t));
-    return t;
-}
-
 // Grid barrier (all CTAs co-resident: cooperative launch).  bar[0] arrivals,
 // bar[1] generation.  A wait longer than WAIT_NS sets *err and every CTA leaves.
 __device__ bool grid_sync(unsigned *bar, int *err, unsigned nblocks)
@@ -422,733 +413,6 @@ __global__ void __launch_bounds__(128) ypass2_kernel(int m, const double *__rest
 }
 
 constexpr int YP1_SMEM = 2 * 128 * (NB + 1) * (int)sizeof(double);
-
-// AB[d + 2NB c] = A(c + d, c), d < 2NB (rows beyond the band zero: room for the bulges)
-__global__ void band_extract_kernel(int n, const double *__restrict__ A, long lda, double *AB)
-{
-    const long idx = blockIdx.x * (long)blockDim.x + threadIdx.x;
-    if (idx >= (long)n * 2 * NB) return;
-    const int d = (int)(idx % (2 * NB)), c = (int)(idx / (2 * NB));
-    AB[idx] = (d <= NB && c + d < n) ? A[(c + d) + lda * (long)c] : 0.0;
-}
-
-// ---------------------------------------------------------------------------
-// stage 2: band -> tridiagonal (bulge chasing)
-// ---------------------------------------------------------------------------
-// Band storage: A(r, c), r >= c, r - c < 2NB, at AB[(r - c) + 2NB c] (the NB rows
-// below the band hold the bulges).  Sweep j annihilates column j below the
-// subdiagonal and chases the bulge: task (j, i) has the window rows
-// r0 = j + 1 + i NB .. r1 = min(r0 + NB, n) - 1 and reduces column col (= j for
-// i = 0, the previous window's first column otherwise) with one reflector H,
-// applied from the left to the rest of the previous bulge (columns col+1..r0-1),
-// from both sides to the diagonal block, and from the right to the NB rows
-// below the window (creating the next bulge).  Task (j, i) may run once sweep
-// j-1 has completed step i+2 (their footprints are disjoint from then on).
-constexpr int LDAB = 2 * NB;
-
-__host__ __device__ __forceinline__ int sweep_steps(int n, int j) { return j <= n - 3 ? (n - 3 - j) / NB + 1 : 0; }
-
-struct Sb2stArgs {
-    double *AB;
-    int n;
-    double *V2;        // reflectors: V2[((long)j * S + i) * NB + t]
-    double *tau2;      // tau2[(long)j * S + i]
-    int S;
-    int *progress;     // completed steps per sweep (zero on entry)
-    int *err;
-};
-
-// one warp per worker CTA; workers take sweeps j = blockIdx.x, + gridDim.x, ...
-__global__ void __launch_bounds__(32) sb2st_kernel(Sb2stArgs a)
-{
-    __shared__ double Lb[NB][NB + 1], Ds[NB][NB + 1], Bs[NB][NB + 1];
-    __shared__ double vs[NB], ws_[NB];
-    const int t = threadIdx.x, n = a.n;
-    double *AB = a.AB;
-    auto at = [&](int r, int c) -> double * { return AB + (r - c) + (long)LDAB * c; };
-    for (int j = blockIdx.x; j < n - 2; j += gridDim.x) {
-        const int nst = sweep_steps(n, j);
-        const int nprev = j > 0 ? sweep_steps(n, j - 1) : 0;
-        for (int i = 0; i < nst; i++) {
-            if (j > 0) {
-                const int need = min(i + 3, nprev);
-                if (t == 0) {
-                    volatile int *pg = a.progress + (j - 1);
-                    const unsigned long long t0 = gtime();
-                    while (*pg < need) {
-                        if (*(volatile int *)a.err) break;
-                        if (gtime() - t0 > WAIT_NS) { atomicExch(a.err, 2); break; }
-                    }
-                    __threadfence();
-                }
-                __syncwarp();
-                if (*(volatile int *)a.err) return;
-            }
-            const int r0 = j + 1 + i * NB, r1 = min(r0 + NB, n), L = r1 - r0;
-            const int col = i == 0 ? j : r0 - NB;
-            const int nl = r0 - col - 1;                        // left columns col+1 .. r0-1
-            const int r2 = min(r1 + NB, n), nb2 = r2 - r1;      // rows below the window
-            // ---- loads (through L2: other workers write the band), every load of a block
-            // issued before any is used so their latencies overlap ----
-            const double x = t < L ? __ldcg(at(r0 + t, col)) : 0.0;
-            {
-                double rl[NB - 1], rd[NB], rb[NB];
-#pragma unroll
-                for (int c = 0; c < NB - 1; c++) rl[c] = (c < nl && t < L) ? __ldcg(at(r0 + t, col + 1 + c)) : 0.0;
-#pragma unroll
-                for (int a2 = 0; a2 < NB; a2++) rd[a2] = (a2 < L && t < L && a2 >= t) ? __ldcg(at(r0 + a2, r0 + t)) : 0.0;
-#pragma unroll
-                for (int q = 0; q < NB; q++) rb[q] = (q < nb2 && t < L) ? __ldcg(at(r1 + q, r0 + t)) : 0.0;
-#pragma unroll
-                for (int c = 0; c < NB - 1; c++) Lb[t][c] = rl[c];
-#pragma unroll
-                for (int a2 = 0; a2 < NB; a2++) Ds[a2][t] = rd[a2];
-#pragma unroll
-                for (int q = 0; q < NB; q++) Bs[q][t] = rb[q];
-            }
-            // ---- the reflector ----
-            double sig = (t >= 1 && t < L) ? x * x : 0.0;
-            for (int o = 16; o > 0; o >>= 1) sig += __shfl_xor_sync(0xffffffffu, sig, o);
-            const double alpha = __shfl_sync(0xffffffffu, x, 0);
-            double tau = 0.0, scale = 0.0, beta = alpha;
-            if (sig != 0.0) {
-                beta = -copysign(sqrt(alpha * alpha + sig), alpha);
-                tau = (beta - alpha) / beta;
-                scale = 1.0 / (alpha - beta);
-            }
-            const double v = t == 0 ? 1.0 : (t < L ? x * scale : 0.0);
-            vs[t] = v;
-            a.V2[((long)j * a.S + i) * NB + t] = v;
-            if (t == 0) a.tau2[(long)j * a.S + i] = tau;
-            if (t < L) *at(r0 + t, col) = t == 0 ? beta : 0.0;
-            __syncwarp();
-            if (tau != 0.0) {
-                // left: columns col+1 .. r0-1 of the window rows (lane = column)
-                if (t < nl) {
-                    double w = 0.0;
-                    for (int q = 0; q < L; q++) w += vs[q] * Lb[q][t];
-                    for (int q = 0; q < L; q++) Lb[q][t] -= tau * vs[q] * w;
-                }
-                // two-sided on the diagonal block: p = tau D v, w = p - tau/2 (v^T p) v
-                double p = 0.0;
-                if (t < L)
-                    for (int b = 0; b < L; b++) p += (t >= b ? Ds[t][b] : Ds[b][t]) * vs[b];
-                p *= tau;
-                double vp = v * p;
-                for (int o = 16; o > 0; o >>= 1) vp += __shfl_xor_sync(0xffffffffu, vp, o);
-                ws_[t] = p - 0.5 * tau * vp * v;
-                __syncwarp();
-                if (t < L)
-                    for (int a2 = t; a2 < L; a2++) Ds[a2][t] -= vs[a2] * ws_[t] + ws_[a2] * vs[t];
-                // right: rows below the window (lane = row)
-                if (t < nb2) {
-                    double sr = 0.0;
-                    for (int c = 0; c < L; c++) sr += Bs[t][c] * vs[c];
-                    for (int c = 0; c < L; c++) Bs[t][c] -= tau * sr * vs[c];
-                }
-                __syncwarp();
-                // ---- stores ----
-                for (int c = 0; c < nl; c++)
-                    if (t < L) *at(r0 + t, col + 1 + c) = Lb[t][c];
-                for (int a2 = 0; a2 < L; a2++)
-                    if (t < L && a2 >= t) *at(r0 + a2, r0 + t) = Ds[a2][t];
-                for (int q = 0; q < nb2; q++)
-                    if (t < L) *at(r1 + q, r0 + t) = Bs[q][t];
-            }
-            __threadfence();
-            __syncwarp();
-            if (t == 0) *(volatile int *)(a.progress + j) = i + 1;
-        }
-    }
-}
-
-// The same tasks with every block held row-wise in registers (lane = row, so the
-// band is read and written coalesced), the reductions across rows through shared
-// memory, and the x column and left block of step i > 0 taken from step i-1's
-// updated lower block (the same rows and columns; no other sweep writes them in
-// between: sweep j-1 is at least three steps ahead, sweep j+1 behind).
-// K warps per CTA: CTA b takes the groups of K consecutive sweeps g = b, b + gridDim.x, ...,
-// warp w sweep g K + w.  A warp waits for its predecessor sweep through a counter in shared
-// memory when the predecessor is a warp of the same CTA (w > 0) and through the global
-// progress array otherwise; the band itself is exchanged through global memory (L2) as before.
-constexpr int SB_WSM = 2 * NB * (NB + 1) + 2 * NB;       // doubles of shared memory per warp
-
-template <int K>
-__global__ void __launch_bounds__(32 * K) sb2st2_kernel(Sb2stArgs a)
-{
-    extern __shared__ __align__(16) double sbsm[];
-    __shared__ volatile int sprog[K];          // it * 4096 + completed steps of warp w's sweep
-    const int t = threadIdx.x & 31, w = threadIdx.x >> 5, n = a.n;
-    double (*Ts)[NB + 1] = (double (*)[NB + 1])(sbsm + w * SB_WSM);            // transpose of D
-    double (*Cs)[NB + 1] = (double (*)[NB + 1])(sbsm + w * SB_WSM + NB * (NB + 1));   // carried block
-    double *vs = sbsm + w * SB_WSM + 2 * NB * (NB + 1), *ws2 = vs + NB;
-    double *AB = a.AB;
-    if (threadIdx.x < K) sprog[threadIdx.x] = 0;
-    __syncthreads();
-    int it = 0;
-    auto at = [&](int r, int c) -> double * { return AB + (r - c) + (long)LDAB * c; };
-    // wait until sweep j-1 has completed `need` steps (bounded; false: give up, the flag is set)
-    auto wait_prev = [&](int j, int need) -> bool {
-        if (j > 0 && need > 0) {
-            if (t == 0) {
-                const unsigned long long t0 = gtime();
-                if (w > 0) {
-                    const int target = it * 4096 + need;
-                    while (sprog[w - 1] < target) {
-                        if (*(volatile int *)a.err) break;
-                        if (gtime() - t0 > WAIT_NS) { atomicExch(a.err, 2); break; }
-                    }
-                } else {
-                    volatile int *pg = a.progress + (j - 1);
-                    while (*pg < need) {
-                        if (*(volatile int *)a.err) break;
-                        if (gtime() - t0 > WAIT_NS) { atomicExch(a.err, 2); break; }
-                    }
-                }
-                __threadfence();
-            }
-            __syncwarp();
-            if (*(volatile int *)a.err) return false;
-        }
-        return true;
-    };
-    // the diagonal and lower blocks of step i of sweep j, lane = row
-    auto load_blocks = [&](int j, int i, double *Dr, double *Br) {
-        const int r0 = j + 1 + i * NB, r1 = min(r0 + NB, n), L = r1 - r0;
-        const int r2 = min(r1 + NB, n), nb2 = r2 - r1;
-#pragma unroll
-        for (int c = 0; c < NB; c++) Dr[c] = (t < L && c <= t) ? __ldcg(at(r0 + t, r0 + c)) : 0.0;
-#pragma unroll
-        for (int c = 0; c < NB; c++) Br[c] = (t < nb2 && c < L) ? __ldcg(at(r1 + t, r0 + c)) : 0.0;
-    };
-    for (int g = blockIdx.x; g * K < n - 2; g += gridDim.x, it++) {
-        const int j = g * K + w;
-        if (j >= n - 2) break;
-        const int nst = sweep_steps(n, j);
-        const int nprev = j > 0 ? sweep_steps(n, j - 1) : 0;
-        double Dr[NB], Br[NB];
-        if (!wait_prev(j, min(3, nprev))) return;
-        load_blocks(j, 0, Dr, Br);
-        for (int i = 0; i < nst; i++) {
-            const int r0 = j + 1 + i * NB, r1 = min(r0 + NB, n), L = r1 - r0;
-            const int col = i == 0 ? j : r0 - NB;
-            const int nl = r0 - col - 1;
-            const int r2 = min(r1 + NB, n), nb2 = r2 - r1;
-            // the blocks of this step were loaded at the end of the previous one (or above)
-            const double xl = i == 0 ? (t < L ? __ldcg(at(r0 + t, col)) : 0.0) : Cs[t][0];
-            // ---- the reflector ----
-            double sig = (t >= 1 && t < L) ? xl * xl : 0.0;
-            for (int o = 16; o > 0; o >>= 1) sig += __shfl_xor_sync(0xffffffffu, sig, o);
-            const double alpha = __shfl_sync(0xffffffffu, xl, 0);
-            double tau = 0.0, scale = 0.0, beta = alpha;
-            if (sig != 0.0) {
-                beta = -copysign(sqrt(alpha * alpha + sig), alpha);
-                tau = (beta - alpha) / beta;
-                scale = 1.0 / (alpha - beta);
-            }
-            const double v = t == 0 ? 1.0 : (t < L ? xl * scale : 0.0);
-            vs[t] = v;
-            a.V2[((long)j * a.S + i) * NB + t] = v;
-            if (t == 0) a.tau2[(long)j * a.S + i] = tau;
-            if (t < L) *at(r0 + t, col) = t == 0 ? beta : 0.0;
-            __syncwarp();
-            if (tau != 0.0) {
-                // left: columns col+1 .. r0-1 = columns 1.. of the carried block; w_c across rows
-                if (nl > 0) {
-                    if (t < nl) {
-                        double w0 = 0.0, w1 = 0.0;
-#pragma unroll
-                        for (int q = 0; q < NB; q += 2) {
-                            w0 = fma(vs[q], Cs[q][t + 1], w0);
-                            w1 = fma(vs[q + 1], Cs[q + 1][t + 1], w1);
-                        }
-                        ws2[t] = tau * (w0 + w1);
-                    }
-                    __syncwarp();
-                    if (t < L) {
-#pragma unroll
-                        for (int c = 0; c < NB - 1; c++)
-                            if (c < nl) *at(r0 + t, col + 1 + c) = fma(-v, ws2[c], Cs[t][c + 1]);
-                    }
-                    __syncwarp();
-                }
-                // two-sided on the diagonal block: p = tau D v, w = p - tau/2 (v^T p) v
-#pragma unroll
-                for (int c = 0; c < NB; c++) Ts[t][c] = Dr[c];
-                __syncwarp();
-                double p0 = 0.0, p1 = 0.0;
-#pragma unroll
-                for (int c = 0; c < NB; c += 2) {
-                    const double d0 = c <= t ? Dr[c] : Ts[c][t];           // D(t, c) from the lower triangle
-                    const double d1 = c + 1 <= t ? Dr[c + 1] : Ts[c + 1][t];
-                    p0 = fma(d0, vs[c], p0);
-                    p1 = fma(d1, vs[c + 1], p1);
-                }
-                const double p = t < L ? tau * (p0 + p1) : 0.0;
-                double vp = v * p;
-                for (int o = 16; o > 0; o >>= 1) vp += __shfl_xor_sync(0xffffffffu, vp, o);
-                const double w = p - 0.5 * tau * vp * v;
-                ws2[t] = w;
-                __syncwarp();
-#pragma unroll
-                for (int c = 0; c < NB; c++)
-                    if (c <= t) Dr[c] -= v * ws2[c] + w * vs[c];
-                // right: rows below the window, s_q = sum_c B(q, c) v_c
-                double s0 = 0.0, s1 = 0.0;
-#pragma unroll
-                for (int c = 0; c < NB; c += 2) {
-                    s0 = fma(Br[c], vs[c], s0);
-                    s1 = fma(Br[c + 1], vs[c + 1], s1);
-                }
-                const double sr = tau * (s0 + s1);
-#pragma unroll
-                for (int c = 0; c < NB; c++) Br[c] = fma(-sr, vs[c], Br[c]);
-                // ---- stores, lane = row ----
-                if (t < L) {
-#pragma unroll
-                    for (int c = 0; c < NB; c++)
-                        if (c <= t) *at(r0 + t, r0 + c) = Dr[c];
-                }
-                if (t < nb2) {
-#pragma unroll
-                    for (int c = 0; c < NB; c++)
-                        if (c < L) *at(r1 + t, r0 + c) = Br[c];
-                }
-            }
-            // the next window's x column and left block are this step's lower block
-#pragma unroll
-            for (int c = 0; c < NB; c++) Cs[t][c] = Br[c];
-            // the next step's blocks (written by nobody in this step; sweep j-1 must be three steps
-            // ahead of it) are requested before this step's stores are fenced, so the two overlap
-            if (i + 1 < nst) {
-                if (!wait_prev(j, min(i + 4, nprev))) return;
-                load_blocks(j, i + 1, Dr, Br);
-            }
-            __threadfence();
-            __syncwarp();
-            if (t == 0) {
-                *(volatile int *)(a.progress + j) = i + 1;
-                sprog[w] = it * 4096 + i + 1;
-            }
-        }
-    }
-}
-
-// The register form with a helper warp: warp 0 computes and stores each step, warp 1 publishes
-// the step (fence, then the progress counter) and polls the previous sweep's counter, so that
-// neither the release fence nor the poll's round trip to L2 sits between two steps of warp 0.
-// Warp 0 hands a step over through the shared counter `done` after a block-scope fence; warp 1
-// observes it, and its device-scope fence orders warp 0's stores before the progress counter
-// (the fence is cumulative over what warp 1 has observed).  The previous sweep's progress goes
-// the other way: warp 1 reads it, fences, and posts it in `seen`.  (A sleep between polls, of
-// even 8 ns, measured slower: the sleep's granularity is coarse.)
-__global__ void __launch_bounds__(64) sb2st3_kernel(Sb2stArgs a)
-{
-    __shared__ double Ts[NB][NB + 1], Cs[NB][NB + 1];
-    __shared__ double vs[NB], ws2[NB];
-    __shared__ volatile int done, seen, quit;
-    const int t = threadIdx.x & 31, w = threadIdx.x >> 5, n = a.n;
-    double *AB = a.AB;
-    auto at = [&](int r, int c) -> double * { return AB + (r - c) + (long)LDAB * c; };
-    for (int j = blockIdx.x; j < n - 2; j += gridDim.x) {
-        const int nst = sweep_steps(n, j);
-        const int nprev = j > 0 ? sweep_steps(n, j - 1) : 0;
-        if (threadIdx.x == 0) { done = 0; seen = j > 0 ? 0 : 1 << 30; quit = 0; }
-        __syncthreads();
-        if (w == 1) {
-            // ---- helper: publish warp 0's steps, watch the previous sweep ----
-            if (t == 0) {
-                int pub = 0, sv = j > 0 ? 0 : 1 << 30;
-                unsigned long long t0 = gtime();
-                while (pub < nst) {
-                    const int d = done;
-                    if (d > pub) {
-                        __threadfence();
-                        *(volatile int *)(a.progress + j) = d;
-                        pub = d;
-                        t0 = gtime();
-                        continue;
-                    }
-                    if (quit) break;
-                    if (sv < nprev) {
-                        const int v = *(volatile int *)(a.progress + (j - 1));
-                        if (v > sv) {
-                            __threadfence();
-                            sv = v;
-                            seen = v;
-                            t0 = gtime();
-                            continue;
-                        }
-                    }
-                    if (*(volatile int *)a.err) { quit = 1; break; }
-                    if (gtime() - t0 > WAIT_NS) { atomicExch(a.err, 2); quit = 1; break; }
-                }
-            }
-            __syncthreads();
-            if (*(volatile int *)a.err) return;
-            continue;
-        }
-        // ---- warp 0: the steps ----
-        // wait until the helper has seen the previous sweep complete `need` steps
-        auto wait_prev = [&](int need) -> bool {
-            if (t == 0) {
-                const unsigned long long t0 = gtime();
-                while (seen < need) {
-                    if (quit) break;
-                    if (gtime() - t0 > WAIT_NS) { atomicExch(a.err, 2); quit = 1; break; }
-                }
-                __threadfence_block();
-            }
-            __syncwarp();
-            return !quit;
-        };
-        auto load_blocks = [&](int i, double *Dr, double *Br) {
-            const int r0 = j + 1 + i * NB, r1 = min(r0 + NB, n), L = r1 - r0;
-            const int r2 = min(r1 + NB, n), nb2 = r2 - r1;
-#pragma unroll
-            for (int c = 0; c < NB; c++) Dr[c] = (t < L && c <= t) ? __ldcg(at(r0 + t, r0 + c)) : 0.0;
-#pragma unroll
-            for (int c = 0; c < NB; c++) Br[c] = (t < nb2 && c < L) ? __ldcg(at(r1 + t, r0 + c)) : 0.0;
-        };
-        double Dr[NB], Br[NB];
-        bool ok = wait_prev(min(3, nprev));
-        if (ok) load_blocks(0, Dr, Br);
-        for (int i = 0; ok && i < nst; i++) {
-            const int r0 = j + 1 + i * NB, r1 = min(r0 + NB, n), L = r1 - r0;
-            const int col = i == 0 ? j : r0 - NB;
-            const int nl = r0 - col - 1;
-            const int r2 = min(r1 + NB, n), nb2 = r2 - r1;
-            const double xl = i == 0 ? (t < L ? __ldcg(at(r0 + t, col)) : 0.0) : Cs[t][0];
-            // ---- the reflector ----
-            double sig = (t >= 1 && t < L) ? xl * xl : 0.0;
-            for (int o = 16; o > 0; o >>= 1) sig += __shfl_xor_sync(0xffffffffu, sig, o);
-            const double alpha = __shfl_sync(0xffffffffu, xl, 0);
-            double tau = 0.0, scale = 0.0, beta = alpha;
-            if (sig != 0.0) {
-                beta = -copysign(sqrt(alpha * alpha + sig), alpha);
-                tau = (beta - alpha) / beta;
-                scale = 1.0 / (alpha - beta);
-            }
-            const double v = t == 0 ? 1.0 : (t < L ? xl * scale : 0.0);
-            vs[t] = v;
-            a.V2[((long)j * a.S + i) * NB + t] = v;
-            if (t == 0) a.tau2[(long)j * a.S + i] = tau;
-            if (t < L) *at(r0 + t, col) = t == 0 ? beta : 0.0;
-            __syncwarp();
-            if (tau != 0.0) {
-                if (nl > 0) {
-                    if (t < nl) {
-                        double w0 = 0.0, w1 = 0.0;
-#pragma unroll
-                        for (int q = 0; q < NB; q += 2) {
-                            w0 = fma(vs[q], Cs[q][t + 1], w0);
-                            w1 = fma(vs[q + 1], Cs[q + 1][t + 1], w1);
-                        }
-                        ws2[t] = tau * (w0 + w1);
-                    }
-                    __syncwarp();
-                    if (t < L) {
-#pragma unroll
-                        for (int c = 0; c < NB - 1; c++)
-                            if (c < nl) *at(r0 + t, col + 1 + c) = fma(-v, ws2[c], Cs[t][c + 1]);
-                    }
-                    __syncwarp();
-                }
-#pragma unroll
-                for (int c = 0; c < NB; c++) Ts[t][c] = Dr[c];
-                __syncwarp();
-                double p0 = 0.0, p1 = 0.0;
-#pragma unroll
-                for (int c = 0; c < NB; c += 2) {
-                    const double d0 = c <= t ? Dr[c] : Ts[c][t];
-                    const double d1 = c + 1 <= t ? Dr[c + 1] : Ts[c + 1][t];
-                    p0 = fma(d0, vs[c], p0);
-                    p1 = fma(d1, vs[c + 1], p1);
-                }
-                const double p = t < L ? tau * (p0 + p1) : 0.0;
-                double vp = v * p;
-                for (int o = 16; o > 0; o >>= 1) vp += __shfl_xor_sync(0xffffffffu, vp, o);
-                const double wv = p - 0.5 * tau * vp * v;
-                ws2[t] = wv;
-                __syncwarp();
-#pragma unroll
-                for (int c = 0; c < NB; c++)
-                    if (c <= t) Dr[c] -= v * ws2[c] + wv * vs[c];
-                double s0 = 0.0, s1 = 0.0;
-#pragma unroll
-                for (int c = 0; c < NB; c += 2) {
-                    s0 = fma(Br[c], vs[c], s0);
-                    s1 = fma(Br[c + 1], vs[c + 1], s1);
-                }
-                const double sr = tau * (s0 + s1);
-#pragma unroll
-                for (int c = 0; c < NB; c++) Br[c] = fma(-sr, vs[c], Br[c]);
-                if (t < L) {
-#pragma unroll
-                    for (int c = 0; c < NB; c++)
-                        if (c <= t) *at(r0 + t, r0 + c) = Dr[c];
-                }
-                if (t < nb2) {
-#pragma unroll
-                    for (int c = 0; c < NB; c++)
-                        if (c < L) *at(r1 + t, r0 + c) = Br[c];
-                }
-            }
-#pragma unroll
-            for (int c = 0; c < NB; c++) Cs[t][c] = Br[c];
-            // hand the step to the helper, then fetch the next step's blocks once the previous sweep
-            // is three steps ahead of it
-            __threadfence_block();
-            __syncwarp();
-            if (t == 0) done = i + 1;
-            if (i + 1 < nst) {
-                ok = wait_prev(min(i + 4, nprev));
-                if (ok) load_blocks(i + 1, Dr, Br);
-            }
-        }
-        if (!ok && t == 0) quit = 1;
-        __syncthreads();
-        if (*(volatile int *)a.err) return;
-    }
-}
-
-// sb2st3_kernel with each step's two-sided update of the diagonal block and its left update of
-// the previous bulge moved to warps of their own (sb2st5_kernel).  Warp 0 keeps the chain from
-// step to step -- the reflector from x, the right update of B, and B's new first column as the
-// next x -- which reads neither.  Warp 2 loads D of step i itself (once the previous sweep has
-// completed step i+2) and updates and stores it; warp 3 applies step i's reflector from the left
-// to the previous step's updated B (warp 0 leaves it in one of two shared buffers) and stores
-// it; both take v_i and tau_i from a ring of four in shared memory and run behind warp 0.  The
-// helper (warp 1) publishes step i once warp 0 has stored step i and warps 2 and 3 step i-1:
-// sweep j+1's step i-2, the first to wait for it, reads the first column of D_{i-1} and of the
-// previous bulge but neither D_i nor step i's left update.  The arithmetic is sb2st3's.
-__global__ void __launch_bounds__(128) sb2st5_kernel(Sb2stArgs a)
-{
-    __shared__ double Ts[NB][NB + 1], Cs[2][NB][NB + 1], Bsm[2][NB][NB + 1];
-    __shared__ double vring[4][NB], tauring[4], ws2[NB], wsd[NB];
-    __shared__ volatile int done, doneD, doneL, vready, bready, seen, quit;
-    const int t = threadIdx.x & 31, w = threadIdx.x >> 5, n = a.n;
-    double *AB = a.AB;
-    auto at = [&](int r, int c) -> double * { return AB + (r - c) + (long)LDAB * c; };
-    // bounded wait of lane 0 until *flag >= need (false: gave up; the error flag is set)
-    auto wait_ge = [&](volatile int *flag, int need) -> bool {
-        if (t == 0) {
-            const unsigned long long t0 = gtime();
-            while (*flag < need) {
-                if (quit) break;
-                if (gtime() - t0 > WAIT_NS) { atomicExch(a.err, 2); quit = 1; break; }
-            }
-            __threadfence_block();
-        }
-        __syncwarp();
-        return !quit;
-    };
-    for (int j = blockIdx.x; j < n - 2; j += gridDim.x) {
-        const int nst = sweep_steps(n, j);
-        const int nprev = j > 0 ? sweep_steps(n, j - 1) : 0;
-        if (threadIdx.x == 0) {
-            done = 0; doneD = 0; doneL = 0; vready = 0; bready = 0; seen = j > 0 ? 0 : 1 << 30; quit = 0;
-        }
-        __syncthreads();
-        if (w == 1) {
-            // ---- helper: publish what both workers have stored, watch the previous sweep ----
-            if (t == 0) {
-                int pub = 0, sv = j > 0 ? 0 : 1 << 30;
-                unsigned long long t0 = gtime();
-                while (pub < nst) {
-                    const int d0 = done, dd = doneD, dl = doneL;
-                    const int ready = (d0 == nst && dd == nst && dl == nst) ? nst
-                                                                          : min(min(d0, min(dd, dl) + 1), nst - 1);
-                    if (ready > pub) {
-                        __threadfence();
-                        *(volatile int *)(a.progress + j) = ready;
-                        pub = ready;
-                        t0 = gtime();
-                        continue;
-                    }
-                    if (quit) break;
-                    if (sv < nprev) {
-                        const int v = *(volatile int *)(a.progress + (j - 1));
-                        if (v > sv) {
-                            __threadfence();
-                            sv = v;
-                            seen = v;
-                            t0 = gtime();
-                            continue;
-                        }
-                    }
-                    if (*(volatile int *)a.err) { quit = 1; break; }
-                    if (gtime() - t0 > WAIT_NS) { atomicExch(a.err, 2); quit = 1; break; }
-                }
-            }
-        } else if (w == 2) {
-            // ---- the diagonal blocks, one step behind warp 0 ----
-            for (int i = 0; i < nst; i++) {
-                const int r0 = j + 1 + i * NB, r1 = min(r0 + NB, n), L = r1 - r0;
-                if (!wait_ge(&seen, min(i + 3, nprev))) break;
-                double Dr[NB];
-#pragma unroll
-                for (int c = 0; c < NB; c++) Dr[c] = (t < L && c <= t) ? __ldcg(at(r0 + t, r0 + c)) : 0.0;
-                if (!wait_ge(&vready, i + 1)) break;
-                const double *vs = vring[i & 3];
-                const double tau = tauring[i & 3], v = vs[t];
-                if (tau != 0.0) {
-#pragma unroll
-                    for (int c = 0; c < NB; c++) Ts[t][c] = Dr[c];
-                    __syncwarp();
-                    double p0 = 0.0, p1 = 0.0;
-#pragma unroll
-                    for (int c = 0; c < NB; c += 2) {
-                        const double d0 = c <= t ? Dr[c] : Ts[c][t];
-                        const double d1 = c + 1 <= t ? Dr[c + 1] : Ts[c + 1][t];
-                        p0 = fma(d0, vs[c], p0);
-                        p1 = fma(d1, vs[c + 1], p1);
-                    }
-                    const double p = t < L ? tau * (p0 + p1) : 0.0;
-                    double vp = v * p;
-                    for (int o = 16; o > 0; o >>= 1) vp += __shfl_xor_sync(0xffffffffu, vp, o);
-                    const double wv = p - 0.5 * tau * vp * v;
-                    wsd[t] = wv;
-                    __syncwarp();
-#pragma unroll
-                    for (int c = 0; c < NB; c++)
-                        if (c <= t) Dr[c] -= v * wsd[c] + wv * vs[c];
-                    if (t < L) {
-#pragma unroll
-                        for (int c = 0; c < NB; c++)
-                            if (c <= t) *at(r0 + t, r0 + c) = Dr[c];
-                    }
-                }
-                __threadfence_block();
-                __syncwarp();
-                if (t == 0) doneD = i + 1;
-            }
-        } else if (w == 3) {
-            // ---- the left updates: step i's reflector on the previous step's updated B; and the
-            //      B block of step i+1 into shared buffer (i+1) & 1 for warp 0, once the previous
-            //      sweep has completed step i+3 ----
-            auto stage_b = [&](int i) -> bool {
-                const int r0 = j + 1 + i * NB, r1 = min(r0 + NB, n), L = r1 - r0;
-                const int r2 = min(r1 + NB, n), nb2 = r2 - r1;
-                if (!wait_ge(&seen, min(i + 3, nprev))) return false;
-                double (*B)[NB + 1] = Bsm[i & 1];
-#pragma unroll
-                for (int c = 0; c < NB; c++) B[t][c] = (t < nb2 && c < L) ? __ldcg(at(r1 + t, r0 + c)) : 0.0;
-                __threadfence_block();
-                __syncwarp();
-                if (t == 0) bready = i + 1;
-                return true;
-            };
-            if (nst > 0 && !stage_b(0)) goto sweep_end;
-            for (int i = 0; i < nst; i++) {
-                const int r0 = j + 1 + i * NB, r1 = min(r0 + NB, n), L = r1 - r0;
-                const int col = i == 0 ? j : r0 - NB;
-                const int nl = r0 - col - 1;
-                if (!wait_ge(&vready, i + 1)) break;
-                const double *vs = vring[i & 3];
-                const double tau = tauring[i & 3], v = vs[t];
-                if (tau != 0.0 && nl > 0) {
-                    double (*C)[NB + 1] = Cs[(i - 1) & 1];
-                    if (t < nl) {
-                        double w0 = 0.0, w1 = 0.0;
-#pragma unroll
-                        for (int q = 0; q < NB; q += 2) {
-                            w0 = fma(vs[q], C[q][t + 1], w0);
-                            w1 = fma(vs[q + 1], C[q + 1][t + 1], w1);
-                        }
-                        ws2[t] = tau * (w0 + w1);
-                    }
-                    __syncwarp();
-                    if (t < L) {
-#pragma unroll
-                        for (int c = 0; c < NB - 1; c++)
-                            if (c < nl) *at(r0 + t, col + 1 + c) = fma(-v, ws2[c], C[t][c + 1]);
-                    }
-                    __syncwarp();
-                }
-                __threadfence_block();
-                __syncwarp();
-                if (t == 0) doneL = i + 1;
-                if (i + 1 < nst && !stage_b(i + 1)) break;
-            }
-        } else {
-            // ---- warp 0: reflectors and right updates ----
-            double Br[NB], xnext = 0.0;
-            bool ok = wait_ge(&seen, min(3, nprev));
-            for (int i = 0; ok && i < nst; i++) {
-                const int r0 = j + 1 + i * NB, r1 = min(r0 + NB, n), L = r1 - r0;
-                const int col = i == 0 ? j : r0 - NB;
-                const int r2 = min(r1 + NB, n), nb2 = r2 - r1;
-                const double xl = i == 0 ? (t < L ? __ldcg(at(r0 + t, col)) : 0.0) : xnext;
-                // ---- the reflector, into ring slot i & 3 once warp 2 has finished step i-4 ----
-                double sig = (t >= 1 && t < L) ? xl * xl : 0.0;
-                for (int o = 16; o > 0; o >>= 1) sig += __shfl_xor_sync(0xffffffffu, sig, o);
-                const double alpha = __shfl_sync(0xffffffffu, xl, 0);
-                double tau = 0.0, scale = 0.0, beta = alpha;
-                if (sig != 0.0) {
-                    beta = -copysign(sqrt(alpha * alpha + sig), alpha);
-                    tau = (beta - alpha) / beta;
-                    scale = 1.0 / (alpha - beta);
-                }
-                const double v = t == 0 ? 1.0 : (t < L ? xl * scale : 0.0);
-                if (i >= 4 && (!(ok = wait_ge(&doneD, i - 3)) || !(ok = wait_ge(&doneL, i - 3)))) break;
-                double *vs = vring[i & 3];
-                vs[t] = v;
-                if (t == 0) tauring[i & 3] = tau;
-                __threadfence_block();                   // (before the global stores: it need not wait for them)
-                __syncwarp();
-                if (t == 0) vready = i + 1;
-                a.V2[((long)j * a.S + i) * NB + t] = v;
-                if (t == 0) a.tau2[(long)j * a.S + i] = tau;
-                if (t < L) *at(r0 + t, col) = t == 0 ? beta : 0.0;
-                if (!(ok = wait_ge(&bready, i + 1))) break;
-                {
-                    const double (*B)[NB + 1] = Bsm[i & 1];
-#pragma unroll
-                    for (int c = 0; c < NB; c++) Br[c] = B[t][c];
-                }
-                if (tau != 0.0) {
-                    double s0 = 0.0, s1 = 0.0;
-#pragma unroll
-                    for (int c = 0; c < NB; c += 2) {
-                        s0 = fma(Br[c], vs[c], s0);
-                        s1 = fma(Br[c + 1], vs[c + 1], s1);
-                    }
-                    const double sr = tau * (s0 + s1);
-#pragma unroll
-                    for (int c = 0; c < NB; c++) Br[c] = fma(-sr, vs[c], Br[c]);
-                    if (t < nb2) {
-#pragma unroll
-                        for (int c = 0; c < NB; c++)
-                            if (c < L) *at(r1 + t, r0 + c) = Br[c];
-                    }
-                }
-                // B goes to buffer i & 1 for warp 3's left update of step i+1, once warp 3 is done
-                // with the buffer's last use (step i-1)
-                xnext = Br[0];
-                if (i >= 1 && !(ok = wait_ge(&doneL, i))) break;
-#pragma unroll
-                for (int c = 0; c < NB; c++) Cs[i & 1][t][c] = Br[c];
-                __threadfence_block();
-                __syncwarp();
-                if (t == 0) done = i + 1;
-            }
-            if (!ok && t == 0) quit = 1;
-        }
-    sweep_end:
-        __syncthreads();
-        if (*(volatile int *)a.err) return;
-    }
-}
-
-// d(c) = A(c, c), e(c) = A(c+1, c)
-__global__ void tridiag_extract_kernel(int n, const double *__restrict__ AB, double *d, double *e)
-{
-    const int c = blockIdx.x * blockDim.x + threadIdx.x;
-    if (c >= n) return;
-    d[c] = AB[(long)LDAB * c];
-    if (c + 1 < n) e[c] = AB[1 + (long)LDAB * c];
-}
 
 // ---------------------------------------------------------------------------
 // back-transformation of the stage-2 reflectors
@@ -2105,7 +1369,7 @@ int symmetrize_lower(int n, const double *A, long lda, double *F, long ldf, cuda
 // The workspace carve-up of syevd2_impl, as offsets (doubles, 32-aligned); the size
 // function and the solver use this one layout.
 struct Syevd2Layout {
-    size_t Wk, AB, V1, T1, V2, tau2, Tq, dv, ev, progress, VYV, X, T, Mp, part, gram, flags, W1, W2, Vg, Gq, Tg,
+    size_t Wk, AB, V1, T1, V2, tau2, Tq, dv, ev, VYV, X, T, Mp, part, gram, flags, W1, W2, Vg, Gq, Tg,
         gemm_ws, dcw, total;
 };
 
@@ -2117,7 +1381,7 @@ static Syevd2Layout syevd2_layout(int n)
     size_t off = 0;
     auto take = [&](size_t cnt) { off = (off + 31) & ~(size_t)31; size_t p = off; off += cnt; return p; };
     L.Wk = take(nn);
-    L.AB = take((size_t)LDAB * n);
+    L.AB = take((size_t)2 * LDAB * n);
     L.V1 = take(sy2sb_vsave_doubles(n));
     L.T1 = take((size_t)(sy2sb_panels(n) + 1) * NB * NB);
     L.V2 = take((size_t)n * S * NB);
@@ -2125,7 +1389,6 @@ static Syevd2Layout syevd2_layout(int n)
     L.Tq = take(ng * S * NB * NB);
     L.dv = take(n);
     L.ev = take(n + 1);
-    L.progress = take(n / 2 + 8);
     L.VYV = take((size_t)n * 6 * NB);               // two [V | Y | V] buffers
     L.X = take((size_t)n * NB);
     L.T = take(NB * NB);
@@ -2164,7 +1427,6 @@ static int syevd2_impl(bsrg_ctx *c, int n, const double *A, long lda, double *w,
     double *Wk = ws + L.Wk, *AB = ws + L.AB, *V1 = ws + L.V1, *T1 = ws + L.T1;
     double *V2 = ws + L.V2, *tau2 = ws + L.tau2, *Tq = ws + L.Tq;
     double *dv = ws + L.dv, *ev = ws + L.ev;
-    int *progress = (int *)(ws + L.progress);
     Sy2sbWork sw;
     sw.VYV = ws + L.VYV;
     sw.VYV2 = sw.VYV + (size_t)n * 3 * NB;
@@ -2185,8 +1447,7 @@ static int syevd2_impl(bsrg_ctx *c, int n, const double *A, long lda, double *w,
     sw.gemm_ws_doubles = 8 * (size_t)Q1W * n;
     sw.gemm_ws = ws + L.gemm_ws;
     double *dcw = ws + L.dcw;
-    if ((e = cudaMemsetAsync(flags, 0, 8 * sizeof(int), st)) != cudaSuccess ||
-        (e = cudaMemsetAsync(progress, 0, sizeof(int) * n, st)) != cudaSuccess)
+    if ((e = cudaMemsetAsync(flags, 0, 8 * sizeof(int), st)) != cudaSuccess)
         return cuda_fail(e, "dsyevd init");
     const int np = sy2sb_panels(n);
     double fl_band = 0.0, fl_chase = 0.0, fl_q2 = 0.0, fl_q1 = 0.0, fl_dc = 0.0;
@@ -2201,56 +1462,16 @@ static int syevd2_impl(bsrg_ctx *c, int n, const double *A, long lda, double *w,
     int rc = symmetrize_lower(n, A, lda, Wk, n, st);
     if (rc == BSRG_OK) rc = sy2sb(st, n, Wk, n, V1, T1, sw);
     if (rc != BSRG_OK) return rc;
-    band_extract_kernel<<<(unsigned)(((long)n * LDAB + 255) / 256), 256, 0, st>>>(n, Wk, n, AB);
+    rc = band_extract(n, Wk, n, AB, st);
+    if (rc != BSRG_OK) return rc;
     stage_end(c, 9, 2 + np * 6);
     c->stage_flops[9] += fl_band;
     stage_begin(c, 10);
     // 2. band -> tridiagonal
-    if (n > 2) {
-        int nsm = 148;
-        cudaDeviceGetAttribute(&nsm, cudaDevAttrMultiProcessorCount, c->device);
-        // the register form with a helper warp (sb2st3_kernel) by default; BSRG_SB2ST_ONEWARP selects the
-        // register form without it, groups of SB_K consecutive sweeps per CTA (sb2st2_kernel<SB_K>), and
-        // BSRG_SB2ST_SHARED the shared-memory form with one sweep per CTA
-        constexpr int SB_K = 1;              // eight sweeps per CTA measured slower (152 vs 121 ms at n = 7810)
-        Sb2stArgs a2{AB, n, V2, tau2, S, progress, sw.err};
-        void *args[] = {&a2};
-        if (!getenv("BSRG_SB2ST_SHARED") && !getenv("BSRG_SB2ST_ONEWARP")) {
-            // one sweep per CTA at a time: the chain of reflectors and right updates on one warp, the
-            // diagonal blocks and the left updates on two more, a helper warp that publishes the steps
-            // (sb2st5_kernel; BSRG_SB2ST_TWOWARP: sb2st3_kernel, computing warp and helper only).  A sweep
-            // starts three steps behind its predecessor, so about sweep_steps / 3 sweeps are active at
-            // once; sweep_steps / 2.5 + 4 CTAs (at most one per SM) never make a sweep wait for its CTA,
-            // and the SMs left over stay free for work on other streams instead of polling
-            // (BSRG_SB2ST_CTAS overrides the count)
-            int want = (int)(sweep_steps(n, 0) / 2.5) + 4;
-            if (const char *ov = getenv("BSRG_SB2ST_CTAS")) want = std::max(1, atoi(ov));
-            const int ctas = std::max(1, std::min(n - 2, std::min(nsm, want)));
-            const bool two = getenv("BSRG_SB2ST_TWOWARP") != nullptr;
-            if ((e = cudaLaunchCooperativeKernel(two ? (const void *)sb2st3_kernel : (const void *)sb2st5_kernel, ctas,
-                                                 two ? 64 : 128, args, 0, st)) != cudaSuccess)
-                return cuda_fail(e, "dsyevd bulge chasing");
-        } else if (getenv("BSRG_SB2ST_SHARED")) {
-            int per = 1;
-            cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per, sb2st_kernel, 32, 0);
-            const int workers = std::max(1, std::min(n - 2, std::min(nsm * std::max(per, 1), 2 * nsm)));
-            if ((e = cudaLaunchCooperativeKernel((const void *)sb2st_kernel, workers, 32, args, 0, st)) != cudaSuccess)
-                return cuda_fail(e, "dsyevd bulge chasing");
-        } else {
-            const int smem = SB_K * SB_WSM * (int)sizeof(double);
-            if ((e = smem_attr(sb2st2_kernel<SB_K>, smem)) !=
-                cudaSuccess)
-                return cuda_fail(e, "dsyevd bulge chasing smem");
-            int per = 1;
-            cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per, sb2st2_kernel<SB_K>, 32 * SB_K, smem);
-            const int groups = (n - 2 + SB_K - 1) / SB_K;
-            const int ctas = std::max(1, std::min(groups, std::min(nsm * std::max(per, 1), 2 * nsm)));
-            if ((e = cudaLaunchCooperativeKernel((const void *)sb2st2_kernel<SB_K>, ctas, 32 * SB_K, args, smem, st)) !=
-                cudaSuccess)
-                return cuda_fail(e, "dsyevd bulge chasing");
-        }
-    }
-    tridiag_extract_kernel<<<(n + 255) / 256, 256, 0, st>>>(n, AB, dv, ev);
+    int nsm = 148;
+    cudaDeviceGetAttribute(&nsm, cudaDevAttrMultiProcessorCount, c->device);
+    rc = bulge_chase(n, AB, dv, ev, V2, tau2, S, sw.err, nsm, st);
+    if (rc != BSRG_OK) return rc;
     for (int j = 0; j < n - 2; j++)
         for (int i = 0; i < sweep_steps(n, j); i++) {
             const double L = std::min(NB, n - (j + 1 + i * NB)), nlf = i == 0 ? 0 : NB - 1;
