@@ -19,6 +19,7 @@ COMMON = ["-O3", "-lineinfo", "-std=c++17", "-Xcompiler", "-fPIC", "-Xcompiler",
 UNITS = {
     "capi.cu": [],
     "rk_tables.cu": ["--fmad=false"],
+    "rk_expand.cu": ["--fmad=false"],
     "convol.cu": ["--fmad=false"],
     "assemble.cu": [],
     "diag_hd.cu": [],

@@ -427,27 +427,12 @@ int bsrg_mtk_cell(const bsrg_basis *b, int k, double fine, double *rkb, int ldp,
     return rc;
 }
 
-// V^k (mode 0) and W^k (mode 1) share the layouts; W^k's moment combinations need a
-// ks*ks*nv scratch, which bsrg_wk_moments allocates and frees
-static int vw_moments_call(const bsrg_basis *b, int k, int mode, double *rkd1, double *rkd2, double *rkd3,
-                           double *rkd4, double *rkd, cudaStream_t s)
-{
-    double *tmp = nullptr;
-    if (mode && (rkd3 || rkd4)) {
-        cudaError_t e = cudaMallocAsync((void **)&tmp, sizeof(double) * (size_t)b->ks * b->ks * b->nv, s);
-        if (e != cudaSuccess) return cuda_fail(e, "wk_moments scratch");
-    }
-    int rc = launch_vw_moments(b, k, mode, rkd1, rkd2, rkd3, rkd4, rkd, tmp, s);
-    if (tmp) cudaFreeAsync(tmp, s);
-    return rc;
-}
-
 int bsrg_vk_moments(const bsrg_basis *b, int k, double *rkd1, double *rkd2, double *rkd3, double *rkd4, double *rkd,
                     void *stream)
 {
     CHECK_ARG(b, "vk_moments: null basis");
     CHECK_ARG(k >= 0 && k <= 64, "vk_moments: k=%d out of range", k);
-    return vw_moments_call(b, k, 0, rkd1, rkd2, rkd3, rkd4, rkd, (cudaStream_t)stream);
+    return launch_vw_moments(b, k, 0, rkd1, rkd2, rkd3, rkd4, rkd, (cudaStream_t)stream);
 }
 
 int bsrg_wk_moments(const bsrg_basis *b, int k, double *rkd1, double *rkd2, double *rkd3, double *rkd4, double *rkd,
@@ -455,7 +440,7 @@ int bsrg_wk_moments(const bsrg_basis *b, int k, double *rkd1, double *rkd2, doub
 {
     CHECK_ARG(b, "wk_moments: null basis");
     CHECK_ARG(k >= 0 && k <= 64, "wk_moments: k=%d out of range", k);
-    return vw_moments_call(b, k, 1, rkd1, rkd2, rkd3, rkd4, rkd, (cudaStream_t)stream);
+    return launch_vw_moments(b, k, 1, rkd1, rkd2, rkd3, rkd4, rkd, (cudaStream_t)stream);
 }
 
 static int mvw_cell_call(const bsrg_basis *b, int k, int mode, double fine, double *rkb, int ldp, cudaStream_t s)
@@ -463,11 +448,10 @@ static int mvw_cell_call(const bsrg_basis *b, int k, int mode, double fine, doub
     const size_t jk = (size_t)b->ks * b->ks, nv = (size_t)b->nv;
     const size_t nj = mode == 2 ? jk : (size_t)ik_of(b->ks);       // pairs on the r2 side
     double *buf = nullptr;
-    cudaError_t e = cudaMallocAsync((void **)&buf, (2 * nj * nv + 3 * jk * nv + jk * nj * nv) * sizeof(double), s);
+    cudaError_t e = cudaMallocAsync((void **)&buf, (2 * nj * nv + 2 * jk * nv + jk * nj * nv) * sizeof(double), s);
     if (e != cudaSuccess) return cuda_fail(e, "m?k_cell scratch");
     double *r1 = buf, *r2 = r1 + nj * nv, *r3 = r2 + nj * nv, *r4 = r3 + jk * nv, *rd = r4 + jk * nv;
-    double *tmp = rd + jk * nj * nv;
-    int rc = launch_vw_moments(b, k, mode, r1, r2, r3, r4, rd, tmp, s);
+    int rc = launch_vw_moments(b, k, mode, r1, r2, r3, r4, rd, s);
     if (rc == BSRG_OK)
         rc = mode == 2 ? launch_mqk_cell(b, r1, r2, r3, r4, rd, fine, rkb, ldp, s)
                        : launch_mvk_cell(b, r1, r2, r3, r4, rd, fine, rkb, ldp, s);
@@ -488,7 +472,7 @@ int bsrg_qk_moments(const bsrg_basis *b, int k, double *rkd1, double *rkd2, doub
 {
     CHECK_ARG(b, "qk_moments: null basis");
     CHECK_ARG(k >= 0 && k <= 64, "qk_moments: k=%d out of range", k);
-    return vw_moments_call(b, k, 2, rkd1, rkd2, rkd3, rkd4, rkd, (cudaStream_t)stream);
+    return launch_vw_moments(b, k, 2, rkd1, rkd2, rkd3, rkd4, rkd, (cudaStream_t)stream);
 }
 
 int bsrg_mqk_cell(const bsrg_basis *b, int k, double fine, double *rkb, int ldp, void *stream)
