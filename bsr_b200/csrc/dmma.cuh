@@ -7,8 +7,12 @@
 // pipeline; every operand tile is staged in shared memory in the orientation
 // its global layout gives (no transposes), with a padding of 4 doubles so that
 // the fragment loads of each half-warp hit 16 distinct 8-byte bank slots.
-// Shapes: 128 x 128 (8 warps, 64 x 32 each) for square work, 128 x 32 and
-// 32 x 128 (4 warps, 32 x 32 each) for the panel products of the eigensolver.
+// Shapes: 64 x 64 (4 warps, 32 x 32 each, three to four CTAs per SM) for square work, 128 x 32 and
+// 32 x 128 (4 warps, 32 x 32 each) for the panel products of the eigensolver.  Several small
+// CTAs fill one another's barriers, prologues and epilogues, and leave a shorter last wave: at
+// 7810^3, 2000 x 820 x 2000 and 1700^3 a 128 x 128 tile of 8 warps took 28.5, 0.272 and 0.464 ms, the
+// 64 x 64 one 27.2, 0.217 and 0.301 (34.6, 0.346 and 0.590 with the slices' copies issued together
+// after the barrier); cuBLAS measures 35.5 TFLOP/s where this is at 35.0.
 //
 // Fragment layouts of m8n8k4 f64 (row.col): A 8x4 -- lane holds A[lane>>2][lane&3];
 // B 4x8 -- lane holds B[lane&3][lane>>2]; C 8x8 -- lane holds C[lane>>2][2(lane&3)+{0,1}].
@@ -31,7 +35,7 @@ template <int BM_, int BN_, int WM_, int WN_> struct Cfg {
     static_assert(TM % 8 == 0 && TN % 8 == 0, "warp tile of whole 8x8 MMA tiles");
     static_assert((BM * BK) % NT == 0 && (BN * BK) % NT == 0, "whole loads per thread");
 };
-using Sq = Cfg<128, 128, 2, 4>;   // 256 threads
+using Sq = Cfg<64, 64, 2, 2>;     // 128 threads
 using Tall = Cfg<128, 32, 4, 1>;  // 128 threads
 using Wide = Cfg<32, 128, 1, 4>;  // 128 threads
 
@@ -43,9 +47,9 @@ template <class C, bool TB> struct BLayout {
     // !TB: Bs[n][k] (k contiguous), TB: Bs[k][n] (n contiguous)
     static constexpr int ELEMS = TB ? BK * (C::BN + PAD) : C::BN * (BK + PAD);
 };
-template <class C, bool TA, bool TB> struct Smem {
+template <class C, bool TA, bool TB, bool SYMA = false> struct Smem {
     static constexpr int STAGE = ALayout<C, TA>::ELEMS + BLayout<C, TB>::ELEMS;
-    static constexpr int BYTES = STAGES * STAGE * 8;
+    static constexpr int BYTES = SYMA ? STAGES * 8 * (ALayout<C, true>::ELEMS + BLayout<C, TB>::ELEMS) : STAGES * STAGE * 8;
 };
 
 __device__ __forceinline__ void cp_async8(double *smem, const double *gmem, bool valid)
@@ -64,97 +68,168 @@ __device__ __forceinline__ void mma884(double &d0, double &d1, double a, double 
                  : "d"(a), "d"(b));
 }
 
-// stage one BK slice of the A and B tiles (zero-filled outside the matrices and
-// outside the K range [k0, kend)).  SYMA: A is square symmetric with only its lower
-// triangle stored; element (m, k) is read from (max, min), a tile wholly above the
-// diagonal with the index order that keeps the reads coalesced.
-template <class C, bool TA, bool TB, bool SYMA = false>
-__device__ __forceinline__ void load_stage(double *sA, double *sB, const double *A, long lda, const double *B,
-                                           long ldb, int M, int N, int kend, int m0, int n0, int k0)
-{
-    const int tid = threadIdx.x;
-    const bool upper_tile = SYMA && m0 + C::BM <= k0;
-#pragma unroll
-    for (int i = 0; i < (C::BM * BK) / C::NT; i++) {
-        const int idx = tid + i * C::NT;
-        int ml, kl;
-        if (!TA && !upper_tile) { ml = idx % C::BM; kl = idx / C::BM; }
-        else { kl = idx % BK; ml = idx / BK; }
-        const int gm = m0 + ml, gk = k0 + kl;
-        const bool v = gm < M && gk < kend;
-        const double *src;
-        if (SYMA) src = v ? (gm >= gk ? A + gm + (long)gk * lda : A + gk + (long)gm * lda) : A;
-        else src = v ? (TA ? A + gk + (long)gm * lda : A + gm + (long)gk * lda) : A;
-        double *dst = TA ? sA + ml * (BK + PAD) + kl : sA + kl * (C::BM + PAD) + ml;
-        cp_async8(dst, src, v);
+// One operand's share of the staging of a BK slice by a thread: N copies, spread over the slice's four
+// MMA steps.  CONTIG elements of the tile are contiguous in memory (m for a column-major A, k for A^T),
+// and a thread's copies differ only along the other index, so a copy costs one pointer addition.
+// Outside the matrix and outside [k0, kend) zeros are staged.
+template <int TILE, bool KFAST, int NT> struct Stager {
+    static constexpr int N = TILE * BK / NT;
+    static constexpr int STEP = KFAST ? NT / BK : NT / TILE;        // tile (or k) indices between two copies
+    static_assert(KFAST ? NT % BK == 0 : NT % TILE == 0, "a thread keeps its contiguous index");
+    static_assert(N % 4 == 0, "whole copies per MMA step");
+    static constexpr int LD = KFAST ? BK + PAD : TILE + PAD;
+    const double *p, *base;
+    long ld, stride;
+    int kl, left, dst;               // first k of this thread in the slice; tile indices it may read (from its first)
+    __device__ __forceinline__ Stager(const double *A, long ld_, int size, int t0, int kbeg, int tid)
+    {
+        const int tl = KFAST ? tid / BK : tid % TILE;
+        kl = KFAST ? tid % BK : tid / TILE;
+        left = size - t0 - tl;
+        base = A;
+        ld = ld_;
+        stride = STEP * ld;
+        p = A + (KFAST ? (kbeg + kl) + (long)(t0 + tl) * ld : (t0 + tl) + (long)(kbeg + kl) * ld);
+        dst = KFAST ? tl * LD + kl : kl * LD + tl;
     }
+    // copies q N / 4 .. of the slice with krem k indices left
+    __device__ __forceinline__ void part(double *s, int q, int krem) const
+    {
 #pragma unroll
-    for (int i = 0; i < (C::BN * BK) / C::NT; i++) {
-        const int idx = tid + i * C::NT;
-        int nl, kl;
-        if (!TB) { kl = idx % BK; nl = idx / BK; }
-        else { nl = idx % C::BN; kl = idx / C::BN; }
-        const int gn = n0 + nl, gk = k0 + kl;
-        const bool v = gn < N && gk < kend;
-        const double *src = v ? (TB ? B + gn + (long)gk * ldb : B + gk + (long)gn * ldb) : B;
-        double *dst = TB ? sB + kl * (C::BN + PAD) + nl : sB + nl * (BK + PAD) + kl;
-        cp_async8(dst, src, v);
+        for (int i = 0; i < N / 4; i++) {
+            const int c = q * (N / 4) + i;
+            const bool v = KFAST ? (kl < krem && c * STEP < left) : (left > 0 && kl + c * STEP < krem);
+            cp_async8(s + dst + c * STEP * LD, v ? p + c * stride : base, v);
+        }
     }
-}
+    __device__ __forceinline__ void advance() { p += KFAST ? BK : BK * ld; }
+};
+
+// The same for a square symmetric A of which only the lower triangle is stored: element (m, k) is read
+// from (max, min), a tile wholly above the diagonal with the index order that keeps the reads coalesced.
+template <int TILE, int NT> struct SymStager {
+    static constexpr int N = TILE * BK / NT, LD = TILE + PAD;
+    const double *base;
+    long ld;
+    int size, t0, k0, tid;
+    __device__ __forceinline__ SymStager(const double *A, long ld_, int size_, int t0_, int kbeg, int tid_)
+        : base(A), ld(ld_), size(size_), t0(t0_), k0(kbeg), tid(tid_)
+    {
+    }
+    __device__ __forceinline__ void part(double *s, int q, int krem) const
+    {
+        const bool upper = t0 + TILE <= k0;
+#pragma unroll
+        for (int i = 0; i < N / 4; i++) {
+            const int idx = tid + (q * (N / 4) + i) * NT;
+            const int tl = upper ? idx / BK : idx % TILE, kl = upper ? idx % BK : idx / TILE;
+            const int gm = t0 + tl, gk = k0 + kl;
+            const bool v = gm < size && kl < krem;
+            cp_async8(s + kl * LD + tl, v ? (gm >= gk ? base + gm + (long)gk * ld : base + gk + (long)gm * ld) : base, v);
+        }
+    }
+    __device__ __forceinline__ void advance() { k0 += BK; }
+};
+template <class C, bool TA, bool SYMA> struct AStager { using T = Stager<C::BM, TA, C::NT>; };
+template <class C, bool TA> struct AStager<C, TA, true> { using T = SymStager<C::BM, C::NT>; };
 
 // acc[s][t][j]: row m0 + wm*TM + s*8 + (lane>>2), column n0 + wn*TN + t*8 + 2*(lane&3) + j,
-// summed over k in [kbeg, kend)
+// summed over k in [kbeg, kend).  The copies of the slice after next are issued a quarter at a time
+// between the MMA steps (issued together after the barrier they left the tensor pipe idle: both warps of a
+// scheduler were in them at once), and a step's fragments are read while the last one's MMAs run.
 template <class C, bool TA, bool TB, bool SYMA = false>
-__device__ __forceinline__ void tile_mma(double (&acc)[C::FM][C::FN][2], double *smem, const double *A, long lda,
+__device__ __forceinline__ void tile_mma_add(double (&acc)[C::FM][C::FN][2], double *smem, const double *A, long lda,
                                          const double *B, long ldb, int M, int N, int kbeg, int kend, int m0, int n0)
 {
     constexpr int SA = ALayout<C, TA>::ELEMS, STG = Smem<C, TA, TB>::STAGE;
     const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
     const int wm = warp % C::WM, wn = warp / C::WM;
     const int r = lane >> 2, c = lane & 3;
-#pragma unroll
-    for (int s = 0; s < C::FM; s++)
-#pragma unroll
-        for (int t = 0; t < C::FN; t++) acc[s][t][0] = acc[s][t][1] = 0.0;
-    const int ktiles = kend > kbeg ? (kend - kbeg + BK - 1) / BK : 0;
+    if (kend <= kbeg) return;
+    const int ktiles = (kend - kbeg + BK - 1) / BK;
+    typename AStager<C, TA, SYMA>::T la(A, lda, M, m0, kbeg, threadIdx.x);
+    Stager<C::BN, !TB, C::NT> lb(B, ldb, N, n0, kbeg, threadIdx.x);
+    int krem = kend - kbeg;
 #pragma unroll
     for (int st = 0; st < STAGES - 1; st++) {
-        if (st < ktiles)
-            load_stage<C, TA, TB, SYMA>(smem + st * STG, smem + st * STG + SA, A, lda, B, ldb, M, N, kend, m0, n0,
-                                        kbeg + st * BK);
-        cp_async_commit();
-    }
-    for (int kt = 0; kt < ktiles; kt++) {
-        cp_async_wait<STAGES - 2>();
-        __syncthreads();
-        const int nk = kt + STAGES - 1;
-        if (nk < ktiles) {
-            double *base = smem + (nk % STAGES) * STG;
-            load_stage<C, TA, TB, SYMA>(base, base + SA, A, lda, B, ldb, M, N, kend, m0, n0, kbeg + nk * BK);
+        if (st < ktiles) {
+#pragma unroll
+            for (int q = 0; q < 4; q++) {
+                la.part(smem + st * STG, q, krem);
+                lb.part(smem + st * STG + SA, q, krem);
+            }
+            la.advance();
+            lb.advance();
+            krem -= BK;
         }
         cp_async_commit();
-        const double *sA = smem + (kt % STAGES) * STG, *sB = sA + SA;
+    }
+    double af[2][C::FM], bf[2][C::FN];
+    auto fragments = [&](int slice, int kk) {
+        const double *sA = smem + (slice % STAGES) * STG, *sB = sA + SA;
+#pragma unroll
+        for (int s = 0; s < C::FM; s++) {
+            const int ml = wm * C::TM + s * 8 + r, kl = kk * 4 + c;
+            af[kk & 1][s] = TA ? sA[ml * (BK + PAD) + kl] : sA[kl * (C::BM + PAD) + ml];
+        }
+#pragma unroll
+        for (int t = 0; t < C::FN; t++) {
+            const int nl = wn * C::TN + t * 8 + r, kl = kk * 4 + c;
+            bf[kk & 1][t] = TB ? sB[kl * (C::BN + PAD) + nl] : sB[nl * (BK + PAD) + kl];
+        }
+    };
+    cp_async_wait<STAGES - 2>();
+    __syncthreads();
+    fragments(0, 0);
+    for (int kt = 0; kt < ktiles; kt++) {
+        const int nk = kt + STAGES - 1;
+        double *next = smem + (nk % STAGES) * STG;
 #pragma unroll
         for (int kk = 0; kk < BK / 4; kk++) {
-            double af[C::FM], bf[C::FN];
-#pragma unroll
-            for (int s = 0; s < C::FM; s++) {
-                const int ml = wm * C::TM + s * 8 + r, kl = kk * 4 + c;
-                af[s] = TA ? sA[ml * (BK + PAD) + kl] : sA[kl * (C::BM + PAD) + ml];
+            if (kk + 1 < BK / 4) fragments(kt, kk + 1);
+            else {
+                // every warp has read the last of this slice: the next one's first fragments before the
+                // last MMAs of this one, so that the barrier is passed with MMAs still to issue
+                cp_async_wait<STAGES - 3>();
+                __syncthreads();
+                fragments(kt + 1, 0);
             }
-#pragma unroll
-            for (int t = 0; t < C::FN; t++) {
-                const int nl = wn * C::TN + t * 8 + r, kl = kk * 4 + c;
-                bf[t] = TB ? sB[kl * (C::BN + PAD) + nl] : sB[nl * (BK + PAD) + kl];
+            if (nk < ktiles) {
+                la.part(next, kk, krem);
+                lb.part(next + SA, kk, krem);
             }
 #pragma unroll
             for (int s = 0; s < C::FM; s++)
 #pragma unroll
-                for (int t = 0; t < C::FN; t++) mma884(acc[s][t][0], acc[s][t][1], af[s], bf[t]);
+                for (int t = 0; t < C::FN; t++) mma884(acc[s][t][0], acc[s][t][1], af[kk & 1][s], bf[kk & 1][t]);
         }
+        la.advance();
+        lb.advance();
+        krem -= BK;
+        cp_async_commit();
     }
     cp_async_wait<0>();
     __syncthreads();
+}
+
+template <class C, bool TA, bool TB, bool SYMA = false>
+__device__ __forceinline__ void tile_mma(double (&acc)[C::FM][C::FN][2], double *smem, const double *A, long lda,
+                                         const double *B, long ldb, int M, int N, int kbeg, int kend, int m0, int n0)
+{
+#pragma unroll
+    for (int s = 0; s < C::FM; s++)
+#pragma unroll
+        for (int t = 0; t < C::FN; t++) acc[s][t][0] = acc[s][t][1] = 0.0;
+    if (!SYMA) {
+        tile_mma_add<C, TA, TB>(acc, smem, A, lda, B, ldb, M, N, kbeg, kend, m0, n0);
+    } else {
+        // left of the diagonal tile A as it is stored, below it A^T: only the tile itself picks its
+        // triangle element by element
+        const int d0 = m0, d1 = m0 + C::BM;
+        tile_mma_add<C, false, TB>(acc, smem, A, lda, B, ldb, M, N, kbeg, min(kend, d0), m0, n0);
+        tile_mma_add<C, false, TB, true>(acc, smem, A, lda, B, ldb, M, N, max(kbeg, d0), min(kend, d1), m0, n0);
+        tile_mma_add<C, true, TB>(acc, smem, A, lda, B, ldb, M, N, max(kbeg, d1), kend, m0, n0);
+    }
 }
 
 }  // namespace dmma

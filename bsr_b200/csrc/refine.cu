@@ -71,19 +71,19 @@ __global__ void __launch_bounds__(dmma::Sq::NT) refine_gemm_kernel(int n, const 
     double acc[C::FM][C::FN][2];
     dmma::tile_mma<C, false, false>(acc, smem, F, ldf, V, ldv, n, n, 0, n, m0, n0);
     const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
-    const int wm = warp & 1, wn = warp >> 1, r = lane >> 2, q = lane & 3;
-    double *red = smem;   // [2 wm][128 columns][3] after the pipeline has drained
+    const int wm = warp % C::WM, wn = warp / C::WM, r = lane >> 2, q = lane & 3;
+    double *red = smem;   // [WM][BN columns][3] after the pipeline has drained
 #pragma unroll
-    for (int t = 0; t < 4; t++)
+    for (int t = 0; t < C::FN; t++)
 #pragma unroll
         for (int j = 0; j < 2; j++) {
-            const int cl = wn * 32 + t * 8 + 2 * q + j, col = n0 + cl;
+            const int cl = wn * C::TN + t * 8 + 2 * q + j, col = n0 + cl;
             double svr = 0.0, srr = 0.0, svv = 0.0;
             if (col < n) {
                 const double lj = lam[col];
 #pragma unroll
-                for (int s = 0; s < 8; s++) {
-                    const int row = m0 + wm * 64 + s * 8 + r;
+                for (int s = 0; s < C::FM; s++) {
+                    const int row = m0 + wm * C::TM + s * 8 + r;
                     if (row < n) {
                         const double v = V[row + (long)ldv * col];
                         const double res = acc[s][t][j] - lj * v;
@@ -101,21 +101,21 @@ __global__ void __launch_bounds__(dmma::Sq::NT) refine_gemm_kernel(int n, const 
                 svv += __shfl_xor_sync(0xffffffffu, svv, o);
             }
             if (r == 0) {
-                red[(wm * 128 + cl) * 3 + 0] = svr;
-                red[(wm * 128 + cl) * 3 + 1] = srr;
-                red[(wm * 128 + cl) * 3 + 2] = svv;
+                red[(wm * C::BN + cl) * 3 + 0] = svr;
+                red[(wm * C::BN + cl) * 3 + 1] = srr;
+                red[(wm * C::BN + cl) * 3 + 2] = svv;
             }
         }
     __syncthreads();
-    for (int idx = threadIdx.x; idx < 128 * 3; idx += C::NT) {
+    for (int idx = threadIdx.x; idx < C::BN * 3; idx += C::NT) {
         const int cl = idx / 3, w = idx % 3, col = n0 + cl;
-        if (col < n) P[((long)blockIdx.x * 3 + w) * n + col] = red[cl * 3 + w] + red[(128 + cl) * 3 + w];
+        if (col < n) P[((long)blockIdx.x * 3 + w) * n + col] = red[cl * 3 + w] + red[(C::BN + cl) * 3 + w];
     }
 }
 
 // The residual epilogue of the mixed-precision form, whose A V comes from the digit product
 // (tc_ozaki.cu) in R: R(i,j) -= lambda_j V(i,j) and the same per-tile partial sums as
-// refine_gemm_kernel, P[(tm*3 + w)*n + j] over rows of 128-row tile tm.  One warp per column
+// refine_gemm_kernel, P[(tm*3 + w)*n + j] over rows of the GEMM's row tile tm.  One warp per column
 // and tile (lanes over rows, shuffles in a fixed order), eight columns per CTA.
 __global__ void __launch_bounds__(256) refine_resid_kernel(int n, const double *__restrict__ V, long ldv,
                                                            const double *__restrict__ lam, double *__restrict__ P,
@@ -126,8 +126,8 @@ __global__ void __launch_bounds__(256) refine_resid_kernel(int n, const double *
     const double lj = lam[col];
     double svr = 0.0, srr = 0.0, svv = 0.0;
 #pragma unroll
-    for (int q = 0; q < 4; q++) {
-        const int row = tm * 128 + q * 32 + lane;
+    for (int q = 0; q < dmma::Sq::BM / 32; q++) {
+        const int row = tm * dmma::Sq::BM + q * 32 + lane;
         if (row < n) {
             const double v = V[row + (long)ldv * col];
             double *rp = R + row + (long)n * col;
@@ -375,7 +375,7 @@ int refine_apply(int n, const double *F, double *V, long ldv, double *lam, doubl
                  int *flag, cudaStream_t s, void *oz_ws, size_t oz_bytes, int *oz_err)
 {
     constexpr int bytes = dmma::Smem<dmma::Sq, false, false>::BYTES;
-    static_assert(bytes >= 2 * 128 * 3 * 8, "epilogue reduction fits the pipeline's shared memory");
+    static_assert(dmma::Sq::WM == 2 && bytes >= 2 * dmma::Sq::BN * 3 * 8, "epilogue reduction fits the pipeline's shared memory");
     cudaError_t e = smem_attr(refine_gemm_kernel, bytes);
     if (e != cudaSuccess) return cuda_fail(e, "refine: shared memory attribute");
     const int ntm = (n + dmma::Sq::BM - 1) / dmma::Sq::BM;
@@ -384,7 +384,6 @@ int refine_apply(int n, const double *F, double *V, long ldv, double *lam, doubl
     double *lamw = Gd + (size_t)RR_ND * n;
     if (oz_ws) {
         // mixed-precision form: A V from 8-bit digits on the tensor cores, then the residual epilogue
-        static_assert(dmma::Sq::BM == 128, "the residual epilogue's tiles are the GEMM's");
         int rc = ozaki_gemm(n, n, n, 1.0, F, n, V, ldv, 0.0, R, n, 8, oz_ws, oz_bytes, oz_err, s);
         if (rc != BSRG_OK) return rc;
         refine_resid_kernel<<<dim3((unsigned)ntm, (unsigned)((n + 7) / 8)), 256, 0, s>>>(n, V, ldv, lam, P, R);
