@@ -30,6 +30,7 @@ UNITS = {
     "refine.cu": [],
     "tridiag_dc.cu": [],
     "syevd2.cu": [],
+    "band_reduce.cu": [],
     "bulge.cu": [],
     "tc_mixed.cu": [],
     "tc_ozaki.cu": [],

@@ -32,388 +32,6 @@
 namespace bsrg {
 namespace {
 
-constexpr int PQ_ROWS = 512;        // panel rows held in shared memory per CTA
-constexpr int PQ_NT = 256;
-// Grid barrier (all CTAs co-resident: cooperative launch).  bar[0] arrivals,
-// bar[1] generation.  A wait longer than WAIT_NS sets *err and every CTA leaves.
-__device__ bool grid_sync(unsigned *bar, int *err, unsigned nblocks)
-{
-    __syncthreads();
-    if (threadIdx.x == 0) {
-        volatile unsigned *vgen = bar + 1;
-        const unsigned my = *vgen;
-        __threadfence();
-        if (atomicAdd(bar, 1u) == nblocks - 1) {
-            atomicExch(bar, 0u);
-            __threadfence();
-            atomicAdd(bar + 1, 1u);
-        } else {
-            const unsigned long long t0 = gtime();
-            while (*vgen == my) {
-                if (*(volatile int *)err) break;
-                if (gtime() - t0 > WAIT_NS) { atomicExch(err, 1); break; }
-            }
-        }
-        __threadfence();
-    }
-    __syncthreads();
-    return *(volatile int *)err == 0;
-}
-
-// ---------------------------------------------------------------------------
-// stage 1: panel QR
-// ---------------------------------------------------------------------------
-struct PanelArgs {
-    double *P;          // panel (m x NB), leading dimension ldp: rows j+NB.., columns j..j+NB-1 of A
-    long ldp;
-    int m, rpc;         // rows, rows per CTA
-    double *V;          // [V | Y | V] buffer (ld m): V written to columns 0..NB-1 and 2NB..3NB-1
-    double *Vs;         // the saved V of this panel for the back-transformation (ld m)
-    double *T;          // NB x NB (ld NB), upper triangular
-    double *Ts;         // saved copy of T
-    double *part;       // per CTA, per column parity: NB dots + NB pivot-row values
-    double *gram;       // per CTA: NB x NB Gram partial
-    unsigned *bar;
-    int *err;
-};
-
-// Householder QR of the panel, LAPACK's dgeqrf/dlarfg conventions:
-// H_c = I - tau_c v_c v_c^T, v_c(c) = 1, P = H_0 ... H_{NB-1} [R; 0].
-__global__ void __launch_bounds__(PQ_NT) panel_qr_kernel(PanelArgs a)
-{
-    extern __shared__ __align__(16) double ps[];       // rpc x (NB + 1)
-    __shared__ double tot[NB], piv[NB], wv[NB], tau_s[NB];
-    __shared__ double sc_tau, sc_scale, sc_beta;
-    const int cta = blockIdx.x, G = gridDim.x, tid = threadIdx.x;
-    const int lane = tid & 31, warp = tid >> 5;
-    const int m = a.m, r0 = cta * a.rpc, nr = max(0, min(a.rpc, m - r0));
-    constexpr int LD = NB + 1;
-    for (int q = tid; q < nr * NB; q += PQ_NT) {
-        const int r = q % nr, c = q / nr;
-        ps[r * LD + c] = a.P[(r0 + r) + a.ldp * (long)c];
-    }
-    const int kb = min(m, NB);
-    __syncthreads();
-    for (int c = 0; c < kb; c++) {
-        double *buf = a.part + ((long)cta * 2 + (c & 1)) * 2 * NB;
-        // partial dots over my rows below the pivot: g_k = sum P(r, c) P(r, k), k >= c
-        for (int k = c + warp; k < NB; k += PQ_NT / 32) {
-            double s = 0.0;
-            for (int r = lane; r < nr; r += 32)
-                if (r0 + r > c) s += ps[r * LD + c] * ps[r * LD + k];
-            for (int o = 16; o > 0; o >>= 1) s += __shfl_xor_sync(0xffffffffu, s, o);
-            if (lane == 0) buf[k] = s;
-        }
-        if (cta == 0)
-            for (int k = c + tid; k < NB; k += PQ_NT) buf[NB + k] = ps[c * LD + k];
-        __threadfence();
-        if (!grid_sync(a.bar, a.err, G)) return;
-        for (int k = c + tid; k < NB; k += PQ_NT) {
-            double s = 0.0;
-            for (int q = 0; q < G; q++) s += __ldcg(a.part + ((long)q * 2 + (c & 1)) * 2 * NB + k);
-            tot[k] = s;
-            piv[k] = __ldcg(a.part + (c & 1) * 2 * NB + NB + k);
-        }
-        __syncthreads();
-        if (tid == 0) {
-            const double alpha = piv[c], sigma = tot[c];
-            if (sigma == 0.0) { sc_tau = 0.0; sc_scale = 0.0; sc_beta = alpha; }
-            else {
-                const double beta = -copysign(sqrt(alpha * alpha + sigma), alpha);
-                sc_tau = (beta - alpha) / beta;
-                sc_scale = 1.0 / (alpha - beta);
-                sc_beta = beta;
-            }
-            tau_s[c] = sc_tau;
-        }
-        __syncthreads();
-        const double tau = sc_tau, scale = sc_scale;
-        for (int k = c + 1 + tid; k < NB; k += PQ_NT) wv[k] = piv[k] + scale * tot[k];   // v^T P(:, k)
-        __syncthreads();
-        // P(:, k) -= tau v w_k, k > c: rows below the pivot, then the pivot row (CTA 0)
-        for (int q = tid; q < nr * (NB - c - 1); q += PQ_NT) {
-            const int r = q % nr, k = c + 1 + q / nr;
-            if (r0 + r > c) ps[r * LD + k] -= tau * scale * ps[r * LD + c] * wv[k];
-        }
-        if (cta == 0)
-            for (int k = c + 1 + tid; k < NB; k += PQ_NT) ps[c * LD + k] -= tau * wv[k];
-        __syncthreads();
-        for (int r = tid; r < nr; r += PQ_NT)
-            if (r0 + r > c) ps[r * LD + c] *= scale;        // v below the pivot
-        if (cta == 0 && tid == 0) ps[c * LD + c] = sc_beta;
-        __syncthreads();
-    }
-    // Gram of V (unit diagonal, zero above), partial over my rows
-    double *gp = a.gram + (long)cta * NB * NB;
-    for (int q = tid; q < NB * NB; q += PQ_NT) {
-        const int i = q % NB, j = q / NB;
-        double s = 0.0;
-        if (i <= j && j < kb)
-            for (int r = 0; r < nr; r++) {
-                const int gr = r0 + r;
-                const double vi = gr > i ? ps[r * LD + i] : (gr == i ? 1.0 : 0.0);
-                const double vj = gr > j ? ps[r * LD + j] : (gr == j ? 1.0 : 0.0);
-                s += vi * vj;
-            }
-        gp[q] = s;
-    }
-    // V out (unit diagonal, zeros above; columns beyond kb are zero) and the band form of the panel
-    for (int q = tid; q < nr * NB; q += PQ_NT) {
-        const int r = q % nr, c = q / nr, gr = r0 + r;
-        const double v = c < kb ? (gr > c ? ps[r * LD + c] : (gr == c ? 1.0 : 0.0)) : 0.0;
-        a.V[gr + (long)m * c] = v;
-        a.V[gr + (long)m * (2 * NB + c)] = v;
-        a.Vs[gr + (long)m * c] = v;
-        a.P[gr + a.ldp * (long)c] = gr <= c ? ps[r * LD + c] : 0.0;
-    }
-    __threadfence();
-    if (!grid_sync(a.bar, a.err, G)) return;
-    if (cta != 0) return;
-    // T from the Gram matrix: T(c,c) = tau_c, T(0:c, c) = -tau_c T(0:c, 0:c) G(0:c, c)
-    double *Gs = ps;                      // reuse: NB x NB
-    for (int q = tid; q < NB * NB; q += PQ_NT) {
-        double s = 0.0;
-        for (int g = 0; g < G; g++) s += __ldcg(a.gram + (long)g * NB * NB + q);
-        Gs[q] = s;
-    }
-    __shared__ double Tt[NB][NB + 1];
-    for (int q = tid; q < NB * NB; q += PQ_NT) Tt[q % NB][q / NB] = 0.0;
-    __syncthreads();
-    for (int c = 0; c < kb; c++) {
-        if (tid < c) {
-            double s = 0.0;
-            for (int l = tid; l < c; l++) s += Tt[tid][l] * Gs[l + NB * c];
-            wv[tid] = s;
-        }
-        __syncthreads();
-        if (tid < c) Tt[tid][c] = -tau_s[c] * wv[tid];
-        if (tid == 0) Tt[c][c] = tau_s[c];
-        __syncthreads();
-    }
-    for (int q = tid; q < NB * NB; q += PQ_NT) {
-        a.T[q] = Tt[q % NB][q / NB];
-        a.Ts[q] = Tt[q % NB][q / NB];
-    }
-}
-
-// The same factorisation on one thread-block cluster (up to 16 CTAs, PQC_ROWS rows each):
-// the per-column partial dot products stay in each CTA's shared memory and are read
-// by every CTA through distributed shared memory after a hardware cluster barrier,
-// instead of a grid barrier over global memory.
-constexpr int PQC_ROWS = 640;
-constexpr int PQC_MAXG = 16;
-
-__global__ void __launch_bounds__(PQ_NT) panel_qr_cluster_kernel(PanelArgs a)
-{
-    namespace cg = cooperative_groups;
-    cg::cluster_group cl = cg::this_cluster();
-    extern __shared__ __align__(16) double ps[];       // rpc x (NB + 1) | partials [2][2 NB] | Gram NB x NB
-    __shared__ double tot[NB], piv[NB], wv[NB], tau_s[NB];
-    __shared__ double sc_tau, sc_scale, sc_beta;
-    const int cta = (int)cl.block_rank(), G = (int)cl.num_blocks(), tid = threadIdx.x;
-    const int lane = tid & 31, warp = tid >> 5;
-    const int m = a.m, r0 = cta * a.rpc, nr = max(0, min(a.rpc, m - r0));
-    constexpr int LD = NB + 1;
-    double *part = ps + (size_t)a.rpc * LD;
-    double *gram = part + 4 * NB;
-    for (int c = warp; c < NB; c += PQ_NT / 32)
-        for (int r = lane; r < nr; r += 32) ps[r * LD + c] = a.P[(r0 + r) + a.ldp * (long)c];
-    const int kb = min(m, NB);
-    __syncthreads();
-    for (int c = 0; c < kb; c++) {
-        double *buf = part + (c & 1) * 2 * NB;
-        for (int k = c + warp; k < NB; k += PQ_NT / 32) {
-            double s = 0.0;
-            for (int r = lane; r < nr; r += 32)
-                if (r0 + r > c) s += ps[r * LD + c] * ps[r * LD + k];
-            for (int o = 16; o > 0; o >>= 1) s += __shfl_xor_sync(0xffffffffu, s, o);
-            if (lane == 0) buf[k] = s;
-        }
-        if (cta == 0)
-            for (int k = c + tid; k < NB; k += PQ_NT) buf[NB + k] = ps[c * LD + k];
-        cl.sync();
-        for (int k = c + tid; k < NB; k += PQ_NT) {
-            double s = 0.0;
-            for (int q = 0; q < G; q++) s += cl.map_shared_rank(buf, q)[k];
-            tot[k] = s;
-            piv[k] = cl.map_shared_rank(buf, 0)[NB + k];
-        }
-        __syncthreads();
-        if (tid == 0) {
-            const double alpha = piv[c], sigma = tot[c];
-            if (sigma == 0.0) { sc_tau = 0.0; sc_scale = 0.0; sc_beta = alpha; }
-            else {
-                const double beta = -copysign(sqrt(alpha * alpha + sigma), alpha);
-                sc_tau = (beta - alpha) / beta;
-                sc_scale = 1.0 / (alpha - beta);
-                sc_beta = beta;
-            }
-            tau_s[c] = sc_tau;
-        }
-        __syncthreads();
-        const double tau = sc_tau, scale = sc_scale;
-        for (int k = c + 1 + tid; k < NB; k += PQ_NT) wv[k] = piv[k] + scale * tot[k];
-        __syncthreads();
-        // a thread per row (stride 33 doubles: conflict-free), columns k > c in registers' reach
-        const double ts_ = tau * scale;
-        for (int r = tid; r < nr; r += PQ_NT) {
-            if (r0 + r <= c) continue;
-            double *row = ps + r * LD;
-            const double f = ts_ * row[c];
-            for (int k = c + 1; k < NB; k++) row[k] -= f * wv[k];
-        }
-        if (cta == 0)
-            for (int k = c + 1 + tid; k < NB; k += PQ_NT) ps[c * LD + k] -= tau * wv[k];
-        __syncthreads();
-        for (int r = tid; r < nr; r += PQ_NT)
-            if (r0 + r > c) ps[r * LD + c] *= scale;
-        if (cta == 0 && tid == 0) ps[c * LD + c] = sc_beta;
-        __syncthreads();
-    }
-    // V in place (unit diagonal, zeros above; columns beyond kb zero), the R part kept aside
-    for (int c = warp; c < NB; c += PQ_NT / 32)
-        for (int r = lane; r < nr; r += 32) {
-            const int gr = r0 + r;
-            const double x = ps[r * LD + c];
-            const double v = c < kb ? (gr > c ? x : (gr == c ? 1.0 : 0.0)) : 0.0;
-            a.V[gr + (long)m * c] = v;
-            a.V[gr + (long)m * (2 * NB + c)] = v;
-            a.Vs[gr + (long)m * c] = v;
-            a.P[gr + a.ldp * (long)c] = gr <= c ? x : 0.0;
-        }
-    __syncthreads();
-    for (int c = warp; c < NB; c += PQ_NT / 32)
-        for (int r = lane; r < nr; r += 32) {
-            const int gr = r0 + r;
-            ps[r * LD + c] = c < kb ? (gr > c ? ps[r * LD + c] : (gr == c ? 1.0 : 0.0)) : 0.0;
-        }
-    __syncthreads();
-    // Gram partial of V over my rows: warp per (i, j) pairs, lanes over rows
-    for (int q = warp; q < NB * NB; q += PQ_NT / 32) {
-        const int i = q % NB, j = q / NB;
-        double sacc = 0.0;
-        if (i <= j)
-            for (int r = lane; r < nr; r += 32) sacc += ps[r * LD + i] * ps[r * LD + j];
-        for (int o = 16; o > 0; o >>= 1) sacc += __shfl_xor_sync(0xffffffffu, sacc, o);
-        if (lane == 0) gram[q] = sacc;
-    }
-    cl.sync();                                          // every CTA's Gram partial is complete
-    if (cta == 0) {
-        __shared__ double Gs[NB * NB];
-        __shared__ double Tt[NB][NB + 1];
-        for (int q = tid; q < NB * NB; q += PQ_NT) {
-            double s = 0.0;
-            for (int g = 0; g < G; g++) s += cl.map_shared_rank(gram, g)[q];
-            Gs[q] = s;
-            Tt[q % NB][q / NB] = 0.0;
-        }
-        __syncthreads();
-        for (int c = 0; c < kb; c++) {
-            if (tid < c) {
-                double s = 0.0;
-                for (int l = tid; l < c; l++) s += Tt[tid][l] * Gs[l + NB * c];
-                wv[tid] = s;
-            }
-            __syncthreads();
-            if (tid < c) Tt[tid][c] = -tau_s[c] * wv[tid];
-            if (tid == 0) Tt[c][c] = tau_s[c];
-            __syncthreads();
-        }
-        for (int q = tid; q < NB * NB; q += PQ_NT) {
-            a.T[q] = Tt[q % NB][q / NB];
-            a.Ts[q] = Tt[q % NB][q / NB];
-        }
-    }
-    cl.sync();                                          // CTA 0 has read every Gram partial
-}
-
-// Y = X T (rows), partial M = V^T Y per chunk of 128 rows.  X, V, Y: ld m.
-__global__ void __launch_bounds__(128) ypass1_kernel(int m, const double *__restrict__ X, const double *__restrict__ V,
-                                                     const double *__restrict__ T, double *Y, double *Mp,
-                                                     unsigned *tick)
-{
-    __shared__ double Ts[NB][NB + 1];
-    extern __shared__ __align__(16) double ysm[];        // Vs, Ys: 128 x (NB + 1) each
-    double (*Vs)[NB + 1] = (double (*)[NB + 1])ysm;
-    double (*Ys)[NB + 1] = (double (*)[NB + 1])(ysm + 128 * (NB + 1));
-    const int tid = threadIdx.x, r0 = blockIdx.x * 128, r = r0 + tid;
-    for (int q = tid; q < NB * NB; q += 128) Ts[q % NB][q / NB] = T[q];
-    __syncthreads();
-    double x[NB];
-#pragma unroll
-    for (int k = 0; k < NB; k++) x[k] = r < m ? X[r + (long)m * k] : 0.0;
-#pragma unroll
-    for (int c = 0; c < NB; c++) {
-        double s = 0.0;
-#pragma unroll
-        for (int k = 0; k < NB; k++) s += x[k] * Ts[k][c];
-        Ys[tid][c] = s;
-        Vs[tid][c] = r < m ? V[r + (long)m * c] : 0.0;
-        if (r < m) Y[r + (long)m * c] = s;
-    }
-    __syncthreads();
-    for (int q = tid; q < NB * NB; q += 128) {
-        const int i = q % NB, j = q / NB;
-        double s0 = 0.0, s1 = 0.0, s2 = 0.0, s3 = 0.0;     // four chains over the rows
-#pragma unroll 4
-        for (int rr = 0; rr < 128; rr += 4) {
-            s0 = fma(Vs[rr][i], Ys[rr][j], s0);
-            s1 = fma(Vs[rr + 1][i], Ys[rr + 1][j], s1);
-            s2 = fma(Vs[rr + 2][i], Ys[rr + 2][j], s2);
-            s3 = fma(Vs[rr + 3][i], Ys[rr + 3][j], s3);
-        }
-        Mp[(long)blockIdx.x * NB * NB + q] = (s0 + s1) + (s2 + s3);
-    }
-    // the last CTA to finish sums the partials in chunk order and forms M2 = 1/2 T^T M once
-    // (at Mp + gridDim.x NB^2) for ypass2; it resets the ticket for the next panel
-    __shared__ unsigned ticket;
-    __threadfence();
-    __syncthreads();
-    if (tid == 0) ticket = atomicAdd(tick, 1u);
-    __syncthreads();
-    if (ticket != gridDim.x - 1) return;
-    __threadfence();
-    double (*Ms)[NB + 1] = Vs;                     // reuse
-    for (int q = tid; q < NB * NB; q += 128) {
-        double s = 0.0;
-        for (int ch = 0; ch < (int)gridDim.x; ch++) s += __ldcg(Mp + (long)ch * NB * NB + q);
-        Ms[q % NB][q / NB] = s;
-    }
-    __syncthreads();
-    double *M2 = Mp + (long)gridDim.x * NB * NB;
-    for (int q = tid; q < NB * NB; q += 128) {
-        const int i = q % NB, j = q / NB;
-        double s = 0.0;
-        for (int l = 0; l <= i; l++) s += Ts[l][i] * Ms[l][j];     // T upper: T^T(i,l) = T(l,i), l <= i
-        M2[q] = 0.5 * s;                                            // column-major M2(i, j)
-    }
-    if (tid == 0) *tick = 0u;
-}
-
-// Y -= V M2 (rows), M2 formed by the last CTA of ypass1
-__global__ void __launch_bounds__(128) ypass2_kernel(int m, const double *__restrict__ V, const double *__restrict__ M2g,
-                                                     double *Y)
-{
-    __shared__ double M2[NB][NB + 1];
-    const int tid = threadIdx.x;
-    for (int q = tid; q < NB * NB; q += 128) M2[q % NB][q / NB] = M2g[q];
-    __syncthreads();
-    const int r = blockIdx.x * 128 + tid;
-    if (r >= m) return;
-    double v[NB];
-#pragma unroll
-    for (int k = 0; k < NB; k++) v[k] = V[r + (long)m * k];
-#pragma unroll
-    for (int c = 0; c < NB; c++) {
-        double s = 0.0;
-#pragma unroll
-        for (int k = 0; k < NB; k++) s += v[k] * M2[k][c];
-        Y[r + (long)m * c] -= s;
-    }
-}
-
-constexpr int YP1_SMEM = 2 * 128 * (NB + 1) * (int)sizeof(double);
-
 // ---------------------------------------------------------------------------
 // back-transformation of the stage-2 reflectors
 // ---------------------------------------------------------------------------
@@ -1177,187 +795,6 @@ __global__ void __launch_bounds__(Q1H) q1_tmerge_kernel(const double *__restrict
 }
 
 }  // namespace
-
-// ---- stage 1 driver ----
-struct Sy2sbWork {
-    double *VYV;       // m x 3NB
-    double *VYV2;      // the second [V | Y | V] buffer (panels alternate while the look-ahead runs)
-    cudaStream_t aux;  // the look-ahead's second stream (null: one stream)
-    cudaEvent_t ev_y, ev_c2;
-    double *X;         // m x NB
-    double *T;         // NB x NB
-    double *Mp;        // chunks x NB x NB
-    double *part;      // PQ CTAs x 4NB
-    double *gram;      // PQ CTAs x NB x NB
-    unsigned *bar;     // 2
-    unsigned *ticket;  // ypass1's last-CTA counter (zero between panels)
-    int *err;
-    double *gemm_ws;   // split-K workspace
-    size_t gemm_ws_doubles;
-};
-
-int sy2sb_panels(int n) { return n > NB ? (n - 1) / NB : 0; }   // panels j = 0, NB, ... with j + NB < n
-
-// Saved panels for the back-transformation: V of panel p (m_p x NB, ld m_p) at Vsave + voff(p),
-// T of panel p at Tsave + p NB^2.
-size_t sy2sb_vsave_doubles(int n)
-{
-    size_t t = 0;
-    for (int j = 0; j + NB < n; j += NB) t += (size_t)(n - j - NB) * NB;
-    return t + 64;
-}
-
-int sy2sb(cudaStream_t st, int n, double *A, long lda, double *Vsave, double *Tsave, const Sy2sbWork &w)
-{
-    cudaError_t e;
-    const int smem = PQ_ROWS * (NB + 1) * (int)sizeof(double);
-    if ((e = smem_attr(panel_qr_kernel, smem)) != cudaSuccess ||
-        (e = smem_attr(ypass1_kernel, YP1_SMEM)) != cudaSuccess)
-        return cuda_fail(e, "sy2sb smem");
-    // the cluster form of the panel factorisation when a 16-CTA cluster with its shared memory fits
-    // (BSRG_PANEL_GRID selects the grid-barrier form)
-    bool use_cluster = !getenv("BSRG_PANEL_GRID");
-    if (use_cluster) {
-        const int smem_c = (PQC_ROWS * (NB + 1) + 4 * NB + NB * NB) * (int)sizeof(double);
-        if (cudaFuncSetAttribute(panel_qr_cluster_kernel, cudaFuncAttributeNonPortableClusterSizeAllowed, 1) !=
-                cudaSuccess ||
-            smem_attr(panel_qr_cluster_kernel, smem_c) !=
-                cudaSuccess) {
-            use_cluster = false;
-        } else {
-            cudaLaunchConfig_t cfg = {};
-            cfg.gridDim = dim3(PQC_MAXG);
-            cfg.blockDim = dim3(PQ_NT);
-            cfg.dynamicSmemBytes = (size_t)smem_c;
-            cudaLaunchAttribute attr[1];
-            attr[0].id = cudaLaunchAttributeClusterDimension;
-            attr[0].val.clusterDim.x = PQC_MAXG;
-            attr[0].val.clusterDim.y = 1;
-            attr[0].val.clusterDim.z = 1;
-            cfg.attrs = attr;
-            cfg.numAttrs = 1;
-            int nclusters = 0;
-            if (cudaOccupancyMaxActiveClusters(&nclusters, panel_qr_cluster_kernel, &cfg) != cudaSuccess ||
-                nclusters < 1)
-                use_cluster = false;
-        }
-        cudaGetLastError();
-    }
-    // factorise panel p (columns j = p NB ..) on stream sq; its V goes to the [V | Y | V] buffer of p's parity
-    auto factor_panel = [&](int p, size_t voff, cudaStream_t sq) -> int {
-        const int j = p * NB, m = n - j - NB;
-        int G = (m + PQ_ROWS - 1) / PQ_ROWS;
-        G = std::max(1, std::min(G, std::max(1, m / NB)));      // CTA 0 holds the NB pivot rows
-        const int rpc = (m + G - 1) / G;
-        if (rpc > PQ_ROWS) { set_error("sy2sb: panel of %d rows does not fit", m); return BSRG_ERR_ARG; }
-        PanelArgs a;
-        a.P = A + (j + NB) + lda * (long)j;
-        a.ldp = lda;
-        a.m = m;
-        a.rpc = rpc;
-        a.V = (p & 1) && w.aux ? w.VYV2 : w.VYV;
-        a.Vs = Vsave + voff;
-        a.T = w.T;
-        a.Ts = Tsave + (size_t)p * NB * NB;
-        a.part = w.part;
-        a.gram = w.gram;
-        a.bar = w.bar;
-        a.err = w.err;
-        const int Gc = std::max(1, (m + PQC_ROWS - 1) / PQC_ROWS);
-        if (use_cluster && Gc <= PQC_MAXG) {
-            // one cluster of Gc CTAs (m / Gc rows each)
-            a.rpc = (m + Gc - 1) / Gc;
-            const int smem_c = (a.rpc * (NB + 1) + 4 * NB + NB * NB) * (int)sizeof(double);
-            cudaLaunchConfig_t cfg = {};
-            cfg.gridDim = dim3((unsigned)Gc);
-            cfg.blockDim = dim3(PQ_NT);
-            cfg.dynamicSmemBytes = (size_t)smem_c;
-            cfg.stream = sq;
-            cudaLaunchAttribute attr[1];
-            attr[0].id = cudaLaunchAttributeClusterDimension;
-            attr[0].val.clusterDim.x = (unsigned)Gc;
-            attr[0].val.clusterDim.y = 1;
-            attr[0].val.clusterDim.z = 1;
-            cfg.attrs = attr;
-            cfg.numAttrs = 1;
-            if ((e = cudaLaunchKernelEx(&cfg, panel_qr_cluster_kernel, a)) != cudaSuccess)
-                return cuda_fail(e, "sy2sb panel (cluster)");
-        } else {
-            void *args[] = {&a};
-            if ((e = cudaLaunchCooperativeKernel((const void *)panel_qr_kernel, G, PQ_NT, args, smem, sq)) !=
-                cudaSuccess)
-                return cuda_fail(e, "sy2sb panel");
-        }
-        return BSRG_OK;
-    };
-    size_t voff = 0;
-    int rc = n > NB ? factor_panel(0, 0, st) : BSRG_OK;
-    if (rc != BSRG_OK) return rc;
-    bool qr_on_aux = false;                       // the current panel was factorised on the aux stream
-    int p = 0;
-    for (int j = 0; j + NB < n; j += NB, p++) {
-        const int m = n - j - NB;
-        double *VYV = (p & 1) && w.aux ? w.VYV2 : w.VYV;
-        double *A22 = A + (j + NB) + lda * (long)(j + NB);
-        double *Vp = VYV, *Yp = VYV + (long)m * NB;
-        const size_t voff_next = voff + (size_t)m * NB;
-        const bool has_next = j + 2 * NB < n;
-        if (qr_on_aux && (e = cudaStreamWaitEvent(st, w.ev_c2, 0)) != cudaSuccess)
-            return cuda_fail(e, "sy2sb look-ahead wait");
-        // X = A22 V with A22 read from its lower triangle (only the lower triangle is updated)
-        DgemmBatch gx{};
-        gx.m = m; gx.n = NB; gx.k = m;
-        gx.A = A22; gx.lda = lda; gx.B = Vp; gx.ldb = m; gx.C = w.X; gx.ldc = m;
-        gx.alpha = 1.0; gx.beta = 0.0; gx.syma = 1;
-        rc = dgemm_ws(false, false, gx, 1, st, w.gemm_ws, w.gemm_ws_doubles);
-        if (rc != BSRG_OK) return rc;
-        const int nch = (m + 127) / 128;
-        ypass1_kernel<<<nch, 128, YP1_SMEM, st>>>(m, w.X, Vp, w.T, Yp, w.Mp, w.ticket);
-        ypass2_kernel<<<nch, 128, 0, st>>>(m, Vp, w.Mp + (size_t)nch * NB * NB, Yp);
-        // A22 -= [V Y] [Y V]^T, the tiles that reach the lower triangle
-        if (!w.aux || m <= NB) {
-            DgemmBatch gu{};
-            gu.m = m; gu.n = m; gu.k = 2 * NB;
-            gu.A = VYV; gu.lda = m; gu.B = Yp; gu.ldb = m; gu.C = A22; gu.ldc = lda;
-            gu.alpha = -1.0; gu.beta = 1.0; gu.lowc = 1;
-            rc = dgemm_ws(false, true, gu, 1, st, nullptr, 0);
-            if (rc == BSRG_OK && has_next) rc = factor_panel(p + 1, voff_next, st);
-            if (rc != BSRG_OK) return rc;
-            qr_on_aux = false;
-        } else {
-            // look-ahead: the next panel's NB columns first; the next panel is then factorised on the
-            // high-priority aux stream while the rest of the trailing matrix is updated here, so the
-            // panel's few CTAs are placed before the update's fill the machine
-            DgemmBatch g1{};
-            g1.m = m; g1.n = NB; g1.k = 2 * NB;
-            g1.A = VYV; g1.lda = m; g1.B = Yp; g1.ldb = m; g1.C = A22; g1.ldc = lda;
-            g1.alpha = -1.0; g1.beta = 1.0;
-            rc = dgemm_ws(false, true, g1, 1, st, nullptr, 0);
-            if (rc != BSRG_OK) return rc;
-            qr_on_aux = false;
-            if (has_next) {
-                if ((e = cudaEventRecord(w.ev_y, st)) != cudaSuccess ||
-                    (e = cudaStreamWaitEvent(w.aux, w.ev_y, 0)) != cudaSuccess)
-                    return cuda_fail(e, "sy2sb look-ahead");
-                rc = factor_panel(p + 1, voff_next, w.aux);
-                if (rc != BSRG_OK) return rc;
-                if ((e = cudaEventRecord(w.ev_c2, w.aux)) != cudaSuccess) return cuda_fail(e, "sy2sb look-ahead");
-                qr_on_aux = true;
-            }
-            const int m2 = m - NB;
-            DgemmBatch g2{};
-            g2.m = m2; g2.n = m2; g2.k = 2 * NB;
-            g2.A = VYV + NB; g2.lda = m; g2.B = Yp + NB; g2.ldb = m; g2.C = A22 + NB + lda * (long)NB; g2.ldc = lda;
-            g2.alpha = -1.0; g2.beta = 1.0; g2.lowc = 1;
-            rc = dgemm_ws(false, true, g2, 1, st, nullptr, 0);
-            if (rc != BSRG_OK) return rc;
-        }
-        voff = voff_next;
-    }
-    if (qr_on_aux && (e = cudaStreamWaitEvent(st, w.ev_c2, 0)) != cudaSuccess)
-        return cuda_fail(e, "sy2sb look-ahead join");
-    return cuda_fail(cudaGetLastError(), "sy2sb");
-}
 
 }  // namespace bsrg
 

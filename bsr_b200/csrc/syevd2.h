@@ -18,6 +18,29 @@ __device__ __forceinline__ unsigned long long gtime()
 // reflectors of sweep j of the bulge chasing
 __host__ __device__ __forceinline__ int sweep_steps(int n, int j) { return j <= n - 3 ? (n - 3 - j) / NB + 1 : 0; }
 
+// stage 1 (band_reduce.cu): the lower triangle of A to a band of width NB in place.  The panels' V go to
+// Vsave one after another (panel p: m_p x NB, m_p = n - (p + 1) NB, ld m_p), their T to Tsave + p NB^2.
+struct Sy2sbWork {
+    double *VYV;       // m x 3NB
+    double *VYV2;      // the second [V | Y | V] buffer (panels alternate while the look-ahead runs)
+    cudaStream_t aux;  // the look-ahead's second stream (null: one stream)
+    cudaEvent_t ev_y, ev_c2;
+    double *X;         // m x NB
+    double *T;         // NB x NB
+    double *Mp;        // chunks x NB x NB
+    double *part;      // PQ CTAs x 4NB
+    double *gram;      // PQ CTAs x NB x NB
+    unsigned *bar;     // 2
+    unsigned *ticket;  // ypass1's last-CTA counter (zero between panels)
+    int *err;
+    double *gemm_ws;   // split-K workspace
+    size_t gemm_ws_doubles;
+};
+
+int sy2sb_panels(int n);
+size_t sy2sb_vsave_doubles(int n);
+int sy2sb(cudaStream_t st, int n, double *A, long lda, double *Vsave, double *Tsave, const Sy2sbWork &w);
+
 // stage 2 (bulge.cu).  band_extract: the band of A (its NB subdiagonals) into AB, 2 LDAB n doubles;
 // bulge_chase: AB to tridiagonal form, d (n) and e (n-1), one cooperative kernel.  Reflector i of
 // sweep j goes to V2[((long)j S + i) NB ..] and tau2[(long)j S + i].  *err (zero on entry) is set to
