@@ -32,6 +32,7 @@ UNITS = {
     "syevd2.cu": [],
     "band_reduce.cu": [],
     "bulge.cu": [],
+    "q2_apply.cu": [],
     "tc_mixed.cu": [],
     "tc_ozaki.cu": [],
     "chan_eig.cu": [],

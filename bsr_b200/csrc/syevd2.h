@@ -49,4 +49,11 @@ int band_extract(int n, const double *A, long lda, double *AB, cudaStream_t s);
 int bulge_chase(int n, double *AB, double *d, double *e, double *V2, double *tau2, int S, int *err, int nsm,
                 cudaStream_t s);
 
+// back-transformation of stage 2 (q2_apply.cu): Z <- Q2 Z for the n columns of Z.  frag:
+// q2_fragment_doubles(n), 16-byte aligned.  *err is set to 3 if a wait runs out.
+size_t q2_fragment_doubles(int n);
+double q2_flops(int n);
+int q2_apply(int n, const double *V2, const double *tau2, int S, double *frag, double *Z, long ldz, int *err, int nsm,
+             cudaStream_t st);
+
 }  // namespace bsrg
