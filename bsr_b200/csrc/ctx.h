@@ -85,7 +85,9 @@ int stage_collect(bsrg_ctx *c);   // waits for recorded events and accumulates
 size_t dc_workspace_bytes(int n);
 size_t dc_pinned_bytes(int n);
 int tridiag_dc(cudaStream_t st, int n, double *d, const double *e, double *w, double *Z, long ldz, void *ws_base,
-               size_t ws_bytes, void *pinned, size_t pinned_bytes, double *gemm_flops, int *launches);
+               size_t ws_bytes, void *pinned, size_t pinned_bytes, int *nmerge, int *launches);
+// the products' operations, once the stream is through with it
+double dc_gemm_flops(int n, void *pinned, int nmerge);
 
 // two-stage dense symmetric eigensolver (syevd2.cu)
 size_t syevd2_workspace_doubles(int n);

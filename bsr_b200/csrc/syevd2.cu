@@ -237,11 +237,10 @@ static int syevd2_impl(bsrg_ctx *c, int n, const double *A, long lda, double *w,
     }
     // 3. tridiagonal eigenpairs into Z
     stage_begin(c, 11);
-    int ndc = 0;
-    rc = tridiag_dc(st, n, dv, ev, w, Z, ldz, dcw, dc_workspace_bytes(n), pinned, pinned_bytes, &fl_dc, &ndc);
+    int ndc = 0, nmerge = 0;
+    rc = tridiag_dc(st, n, dv, ev, w, Z, ldz, dcw, dc_workspace_bytes(n), pinned, pinned_bytes, &nmerge, &ndc);
     if (rc != BSRG_OK) return rc;
     stage_end(c, 11, ndc);
-    c->stage_flops[11] += fl_dc;
     // 4. back-transformation: Q2 then Q1
     stage_begin(c, 12);
     rc = q2_apply(n, V2, tau2, S, Tq, Z, ldz, sw.err, nsm, st);
@@ -298,12 +297,14 @@ static int syevd2_impl(bsrg_ctx *c, int n, const double *A, long lda, double *w,
     }
     stage_end(c, 13, 10 * ((np + Q1_GROUP - 1) / Q1_GROUP));
     c->stage_flops[13] += fl_q1;
-    c->stage_flops[6] += fl_band + fl_chase + fl_dc + fl_q2 + fl_q1;
     // device-side waits report through the flags
     int hflag[2] = {0, 0};
     if ((e = cudaMemcpyAsync(hflag, flags + 2, sizeof(int) * 2, cudaMemcpyDeviceToHost, st)) != cudaSuccess ||
         (e = cudaStreamSynchronize(st)) != cudaSuccess)
         return cuda_fail(e, "dsyevd");
+    fl_dc = dc_gemm_flops(n, pinned, nmerge);
+    c->stage_flops[11] += fl_dc;
+    c->stage_flops[6] += fl_band + fl_chase + fl_dc + fl_q2 + fl_q1;
     if (hflag[0] != 0) {
         set_error("dsyevd: a device-side wait timed out (%s)",
                   hflag[0] == 2 ? "bulge chasing" : hflag[0] == 3 ? "back-transformation wavefront" : "panel barrier");
@@ -351,6 +352,8 @@ extern "C" int bsrg_dsyevd(bsrg_ctx *c, int n, const double *A, int lda, double 
     int rc = ctx_reserve(c, syevd2_workspace_doubles(n) * sizeof(double) + 1024);
     if (rc == BSRG_OK) rc = ctx_reserve_pinned(c, dc_pinned_bytes(n));
     if (rc != BSRG_OK) return rc;
+    cudaError_t e = cudaEventSynchronize(c->ev_stage);     // the staging's last copies are through
+    if (e != cudaSuccess) return cuda_fail(e, "dsyevd staging");
     rc = dense_syevd(c, n, A, lda, w, Z, ldz, (double *)c->ws, c->ws_bytes / sizeof(double), c->pinned,
                      c->pinned_bytes, nullptr);
     cudaEventRecord(c->ev_stage, c->stream);

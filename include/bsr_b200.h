@@ -419,7 +419,7 @@ int bsrg_dsytrd(bsrg_ctx *c, int n, double *A, int lda, double *d, double *e, do
  *      (ascending, w) and eigenvectors (Z, ldz >= n) of the symmetric tridiagonal
  *      T = tridiag(e, d, e) by divide and conquer (LAPACK DSTEDC's algorithm).
  *      d (n), e (n-1) device, unchanged.  n <= 10240.  Uses the context's stream
- *      and workspace; reads small per-level counts back to the host. */
+ *      and workspace. */
 int bsrg_dstedc(bsrg_ctx *c, int n, const double *d, const double *e, double *w, double *Z, int ldz);
 
 /* ---- DSYEV('V','L') as called by LAP_DSYEV (src/libs/ZCOM/LAPACK_calls.f90:54-76,
