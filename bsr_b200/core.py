@@ -368,8 +368,8 @@ class Context:
         call("bsrg_ctx_set_precision", self.handle, {"i8": 1, "tf32": 2}[form] if mixed else 0)
 
     def set_eigensolver(self, which="auto"):
-        """diag_hd's dense eigensolver: "auto" (the library's from 7000 rows, cuSOLVER's below),
-        "own" (the library's two-stage solver) or "lib" (cuSOLVER's syevd)."""
+        """diag_hd's dense eigensolver: "auto" (the library's from 640 rows, without vectors
+        from 256, cuSOLVER's below), "own" (the library's two-stage solver) or "lib" (cuSOLVER's syevd)."""
         call("bsrg_ctx_set_eigensolver", self.handle, {"auto": 0, "own": 1, "lib": 2}[which])
 
     def refine_stats(self, n):

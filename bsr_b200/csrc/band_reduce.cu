@@ -53,7 +53,7 @@ struct PanelArgs {
     long ldp;
     int m, rpc;         // rows, rows per CTA
     double *V;          // [V | Y | V] buffer (ld m): V written to columns 0..NB-1 and 2NB..3NB-1
-    double *Vs;         // the saved V of this panel for the back-transformation (ld m)
+    double *Vs;         // the saved V of this panel for the back-transformation (ld m), or null
     double *T;          // NB x NB (ld NB), upper triangular
     double *Ts;         // saved copy of T
     double *part;       // per CTA, per column parity: NB dots + NB pivot-row values
@@ -149,7 +149,7 @@ __global__ void __launch_bounds__(PQ_NT) panel_qr_kernel(PanelArgs a)
         const double v = c < kb ? (gr > c ? ps[r * LD + c] : (gr == c ? 1.0 : 0.0)) : 0.0;
         a.V[gr + (long)m * c] = v;
         a.V[gr + (long)m * (2 * NB + c)] = v;
-        a.Vs[gr + (long)m * c] = v;
+        if (a.Vs) a.Vs[gr + (long)m * c] = v;
         a.P[gr + a.ldp * (long)c] = gr <= c ? ps[r * LD + c] : 0.0;
     }
     __threadfence();
@@ -178,7 +178,7 @@ __global__ void __launch_bounds__(PQ_NT) panel_qr_kernel(PanelArgs a)
     }
     for (int q = tid; q < NB * NB; q += PQ_NT) {
         a.T[q] = Tt[q % NB][q / NB];
-        a.Ts[q] = Tt[q % NB][q / NB];
+        if (a.Ts) a.Ts[q] = Tt[q % NB][q / NB];
     }
 }
 
@@ -427,7 +427,7 @@ __global__ void __launch_bounds__(PC_NT) panel_qr_cluster_kernel(PanelArgs a)
             const double v = ps[r * PLD + c];
             a.V[(r0 + r) + (long)m * c] = v;
             a.V[(r0 + r) + (long)m * (2 * NB + c)] = v;
-            a.Vs[(r0 + r) + (long)m * c] = v;
+            if (a.Vs) a.Vs[(r0 + r) + (long)m * c] = v;
         }
     if (cta == 0) {
         for (int q = tid; q < NB * NB; q += PC_NT) {
@@ -455,7 +455,7 @@ __global__ void __launch_bounds__(PC_NT) panel_qr_cluster_kernel(PanelArgs a)
         __syncthreads();
         for (int q = tid; q < NB * NB; q += PC_NT) {
             a.T[q] = s.T[q % NB][q / NB];
-            a.Ts[q] = s.T[q % NB][q / NB];
+            if (a.Ts) a.Ts[q] = s.T[q % NB][q / NB];
         }
     }
     cl.sync();                                              // no CTA leaves while another may still write to it
@@ -649,9 +649,9 @@ int sy2sb(cudaStream_t st, int n, double *A, long lda, double *Vsave, double *Ts
         a.m = m;
         a.rpc = rpc;
         a.V = (p & 1) && w.aux ? w.VYV2 : w.VYV;
-        a.Vs = Vsave + voff;
+        a.Vs = Vsave ? Vsave + voff : nullptr;
         a.T = w.T;
-        a.Ts = Tsave + (size_t)p * NB * NB;
+        a.Ts = Tsave ? Tsave + (size_t)p * NB * NB : nullptr;
         a.part = w.part;
         a.gram = w.gram;
         a.bar = w.bar;

@@ -383,8 +383,8 @@ __global__ void __launch_bounds__(BULGE_NT, 1) bulge_kernel(BulgeArgs a)
                     if (t == 0) st_pair(at(n - 1, n - 1), corner[0], after);
                 }
                 const double scale = binv == 0.0 ? 0.0 : 1.0 / u0;
-                a.V2[((long)j * a.S + i) * NB + t] = t == 0 ? 1.0 : (t < L ? u * scale : 0.0);
-                if (t == 0) a.tau2[(long)j * a.S + i] = binv == 0.0 ? 0.0 : 1.0 - alpha * binv;
+                if (a.V2) a.V2[((long)j * a.S + i) * NB + t] = t == 0 ? 1.0 : (t < L ? u * scale : 0.0);
+                if (t == 0 && a.V2) a.tau2[(long)j * a.S + i] = binv == 0.0 ? 0.0 : 1.0 - alpha * binv;
                 __syncwarp();
                 if (t == 0) *(volatile int *)&s.doneD = i + 1;
             }

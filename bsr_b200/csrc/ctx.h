@@ -88,11 +88,14 @@ int tridiag_dc(cudaStream_t st, int n, double *d, const double *e, double *w, do
                size_t ws_bytes, void *pinned, size_t pinned_bytes, int *nmerge, int *launches);
 // the products' operations, once the stream is through with it
 double dc_gemm_flops(int n, void *pinned, int nmerge);
+// the eigenvalues alone, by bisection; work: 8 doubles
+int tridiag_values(cudaStream_t st, int n, const double *d, const double *e, double *w, double *work);
 
 // two-stage dense symmetric eigensolver (syevd2.cu)
-size_t syevd2_workspace_doubles(int n);
+size_t syevd2_workspace_doubles(int n, bool vectors = true);
+// Z null: eigenvalues only (no pinned staging needed); *info = 1: the matrix is not finite, the results are NaN
 int dense_syevd(bsrg_ctx *c, int n, const double *A, long lda, double *w, double *Z, long ldz, double *ws,
-                size_t ws_doubles, void *pinned, size_t pinned_bytes, int *launches);
+                size_t ws_doubles, void *pinned, size_t pinned_bytes, int *launches, int *info);
 
 // the channel eigenproblems of diag_hd (chan_eig.cu)
 bool chan_own_ok(int ns, int ks, int npad, int device);

@@ -368,9 +368,11 @@ static int solve_channels_batched(bsrg_ctx *c, cusolverDnParams_t params, const 
 using namespace bsrg;
 
 // smallest dense problem (by its row bound) for which diag_hd uses the library's eigensolver by
-// default: measured against cuSOLVER's syevd on a B200, 399 vs 421 ms at 7810 rows, 258 vs 228 ms
-// at 6000 and 154 vs 114 ms at 4500
-constexpr int kOwnEigMin = 7000;
+// default, with eigenvectors and without
+// (whole call, library's against cuSOLVER's, ms: with vectors 3.83 / 3.51 at 230 rows, 5.02 / 4.85 at 344,
+// 24.6 / 28.1 at 1564, 68 / 94 at 3907, 239 / 455 at 7810; without 2.94 / 3.17 at 230, 3.92 / 4.42 at 344,
+// 21.5 / 26.1 at 1564, 51 / 81 at 3907, 126 / 380 at 7810)
+constexpr int kOwnEigMin = 640, kOwnValMin = 256;
 
 // scc == NULL: the block-diagonal overlap (diag_ovl /= 0); otherwise the generalized
 // branch with the channel-channel overlap blocks of scc (diag_ovl = 0)
@@ -407,13 +409,13 @@ static int diag_hd_impl(bsrg_ctx *c, const bsrg_basis *b, int nch, const int *lc
     const bool refine = want_vectors && c->refine;
     const char *eig_env = getenv("BSRG_EIG");
     // the library's two-stage eigensolver (syevd2.cu) or cuSOLVER's syevd: BSRG_EIG=own or =lib
-    // chooses, else the context's setting; by default the library's from kOwnEigMin rows up (where
-    // it was measured faster)
+    // chooses, else the context's setting; by default the library's from kOwnEigMin
+    // (kOwnValMin without vectors) rows up, unless its workspace does not fit the device
     int khm_bound = 0;
     for (int ich = 0; ich < nch; ich++) khm_bound += nsolv[ich];
-    const bool own_eig = want_vectors && khm_bound <= 10240 &&
-                         (eig_env ? strcmp(eig_env, "own") == 0
-                                  : (c->eig_mode == 1 || (c->eig_mode == 0 && khm_bound >= kOwnEigMin)));
+    const bool auto_eig = !eig_env && c->eig_mode == 0;
+    bool own_eig = khm_bound <= 10240 && (auto_eig ? khm_bound >= (want_vectors ? kOwnEigMin : kOwnValMin)
+                                                   : eig_env ? strcmp(eig_env, "own") == 0 : c->eig_mode == 1);
     std::vector<BlockMap> bmap;
     for (int ic = 1; ic < nch; ic++)
         for (int jc = 0; jc < ic; jc++) bmap.push_back({ic, jc});
@@ -438,12 +440,10 @@ static int diag_hd_impl(bsrg_ctx *c, const bsrg_basis *b, int nch, const int *lc
     }
     cusolverEigMode_t jobz = want_vectors ? CUSOLVER_EIG_MODE_VECTOR : CUSOLVER_EIG_MODE_NOVECTOR;
     size_t dws = 0, hws = 0;
-    if (cusolverDnXsyevd_bufferSize(c->solver, params, jobz, CUBLAS_FILL_MODE_LOWER, khm_max, CUDA_R_64F, nullptr,
-                                    khm_max, CUDA_R_64F, nullptr, CUDA_R_64F, &dws, &hws) != CUSOLVER_STATUS_SUCCESS) {
-        cusolverDnDestroyParams(params);
-        set_error("diag_hd: syevd_bufferSize failed");
-        return BSRG_ERR_SOLVER;
-    }
+    auto lib_sizes = [&](int n) {
+        return cusolverDnXsyevd_bufferSize(c->solver, params, jobz, CUBLAS_FILL_MODE_LOWER, n, CUDA_R_64F, nullptr, n,
+                                           CUDA_R_64F, nullptr, CUDA_R_64F, &dws, &hws) == CUSOLVER_STATUS_SUCCESS;
+    };
     size_t need = 0;
     auto add = [&](size_t bytes) { need += ((bytes + 255) & ~(size_t)255) + 256; };
     add(sizeof(int) * nch * 3 + 64);      // s0, nsol, counts
@@ -456,7 +456,6 @@ static int diag_hd_impl(bsrg_ctx *c, const bsrg_basis *b, int nch, const int *lc
     add(sizeof(double *) * std::max(nb, 1) * 6);
     add(sizeof(double) * nn * std::max(nb, 1) * 2);   // Wt, T
     if (!vecs) add(sizeof(double) * (size_t)khm_max * khm_max);
-    add(dws + 16);
     // the mixed-precision form's A V from 8-bit digits (its K limit: the FP64 GEMM beyond)
     const bool oz_refine = refine && c->precision == 1 && khm_max <= BSRG_OZAKI_KMAX;
     const size_t oz_bytes = oz_refine ? ozaki_ws_bytes(khm_max, khm_max, khm_max, 8) : 0;
@@ -465,7 +464,6 @@ static int diag_hd_impl(bsrg_ctx *c, const bsrg_basis *b, int nch, const int *lc
         add(sizeof(int) * 4);
         if (oz_refine) add(oz_bytes);
     }
-    if (own_eig) add(sizeof(double) * syevd2_workspace_doubles(khm_max));
     const bool gen = scc != nullptr;
     int nbo = 0;                          // off-diagonal overlap blocks to transform
     if (gen) {
@@ -484,7 +482,19 @@ static int diag_hd_impl(bsrg_ctx *c, const bsrg_basis *b, int nch, const int *lc
         add(sizeof(double) * chan_own_workspace_doubles(nch, npad, ks));
         add(sizeof(int) * 4);
     }
-    int rc = ctx_reserve(c, need);
+    int rc = BSRG_OK;
+    if (own_eig) {
+        rc = ctx_reserve(c, need + sizeof(double) * syevd2_workspace_doubles(khm_max, want_vectors) + 512);
+        if (rc != BSRG_OK && auto_eig) own_eig = false;
+    }
+    if (!own_eig) {
+        if (!lib_sizes(khm_max)) {
+            cusolverDnDestroyParams(params);
+            set_error("diag_hd: syevd_bufferSize failed");
+            return BSRG_ERR_SOLVER;
+        }
+        rc = ctx_reserve(c, need + dws + 528);
+    }
     if (rc != BSRG_OK) { cusolverDnDestroyParams(params); return rc; }
     // pinned staging layout (ints): s0 | nsol | info | cnt | ipsol | final info, then block maps and pointers
     const size_t o_s0 = 0, o_nsol = nch, o_info = 2 * (size_t)nch, o_cnt = 3 * (size_t)nch, o_ip = 4 * (size_t)nch,
@@ -492,7 +502,7 @@ static int diag_hd_impl(bsrg_ctx *c, const bsrg_basis *b, int nch, const int *lc
     size_t o_bm_bytes = ((o_fin + 2) * sizeof(int) + 15) & ~(size_t)15;
     size_t o_ptr_bytes = (o_bm_bytes + sizeof(BlockMap) * nb + 15) & ~(size_t)15;
     const size_t o_dc_bytes = (o_ptr_bytes + sizeof(double *) * nb * 6 + 64 + 255) & ~(size_t)255;
-    rc = ctx_reserve_pinned(c, o_dc_bytes + (own_eig ? dc_pinned_bytes(khm_max) : 0) + 64);
+    rc = ctx_reserve_pinned(c, o_dc_bytes + (own_eig && want_vectors ? dc_pinned_bytes(khm_max) : 0) + 64);
     if (rc != BSRG_OK) { cusolverDnDestroyParams(params); return rc; }
     Arena ar{(char *)c->ws, 0, c->ws_bytes};
     int *d_s0 = ar.take<int>(nch), *d_nsol = ar.take<int>(nch), *d_cnt = ar.take<int>(nch);
@@ -504,11 +514,11 @@ static int diag_hd_impl(bsrg_ctx *c, const bsrg_basis *b, int nch, const int *lc
     double **d_ptrs = ar.take<double *>((size_t)std::max(nb, 1) * 6);
     double *Wt = ar.take<double>(nn * std::max(nb, 1)), *T = ar.take<double>(nn * std::max(nb, 1));
     double *Abuf = vecs ? nullptr : ar.take<double>((size_t)khm_max * khm_max);
-    void *dwork = ar.take<char>(dws + 16);
+    void *dwork = own_eig ? nullptr : ar.take<char>(dws + 16);
     double *Fsym = refine ? ar.take<double>(refine_workspace_doubles(khm_max)) : nullptr;
     int *d_rflag = refine ? ar.take<int>(4) : nullptr;
     char *oz_ws = oz_refine ? ar.take<char>(oz_bytes) : nullptr;
-    double *eig_ws = own_eig ? ar.take<double>(syevd2_workspace_doubles(khm_max)) : nullptr;
+    double *eig_ws = own_eig ? ar.take<double>(syevd2_workspace_doubles(khm_max, want_vectors)) : nullptr;
     double *chan_ws = own_chan ? ar.take<double>(chan_own_workspace_doubles(nch, npad, ks)) : nullptr;
     double *Cov = gen ? ar.take<double>((size_t)khm_max * khm_max) : nullptr;
     double *Tgst = gen ? ar.take<double>((size_t)khm_max * khm_max) : nullptr;
@@ -596,9 +606,7 @@ static int diag_hd_impl(bsrg_ctx *c, const bsrg_basis *b, int nch, const int *lc
         return BSRG_ERR_INFO;
     }
     const size_t dws_cap = dws;
-    if (cusolverDnXsyevd_bufferSize(c->solver, params, jobz, CUBLAS_FILL_MODE_LOWER, khm, CUDA_R_64F, nullptr, khm,
-                                    CUDA_R_64F, nullptr, CUDA_R_64F, &dws, &hws) != CUSOLVER_STATUS_SUCCESS ||
-        dws > dws_cap) {
+    if (!own_eig && (!lib_sizes(khm) || dws > dws_cap)) {
         cusolverDnDestroyParams(params);
         set_error("diag_hd: syevd_bufferSize failed");
         return BSRG_ERR_SOLVER;
@@ -710,11 +718,13 @@ static int diag_hd_impl(bsrg_ctx *c, const bsrg_basis *b, int nch, const int *lc
     stage_begin(c, 6);
     if (own_eig) {
         cusolverDnDestroyParams(params);
-        int nlaunch = 0;
-        int re = dense_syevd(c, khm, A, khm, eval, A, khm, eig_ws, syevd2_workspace_doubles(khm_max),
-                             (char *)c->pinned + o_dc_bytes, c->pinned_bytes - o_dc_bytes, &nlaunch);
+        int nlaunch = 0, eig_info = 0;
+        int re = dense_syevd(c, khm, A, khm, eval, want_vectors ? A : nullptr, khm, eig_ws,
+                             syevd2_workspace_doubles(khm_max, want_vectors),
+                             (char *)c->pinned + o_dc_bytes, c->pinned_bytes - o_dc_bytes, &nlaunch, &eig_info);
         stage_end(c, 6, nlaunch);
         if (re != BSRG_OK) return re;
+        if (eig_info != 0) { set_error("LAP_DSYEV: DSYEV(lapack) gives INFO = %d", eig_info); return BSRG_ERR_INFO; }
         if ((e = cudaMemsetAsync(d_info + nch, 0, sizeof(int), s)) != cudaSuccess) return cuda_fail(e, "diag_hd info");
     } else {
         cusolverStatus_t st = cusolverDnXsyevd(c->solver, params, jobz, CUBLAS_FILL_MODE_LOWER, khm, CUDA_R_64F, A,

@@ -351,13 +351,6 @@ static size_t refine_work_doubles(int n)
 
 size_t refine_workspace_doubles(int n) { return (size_t)n * n + refine_work_doubles(n); }
 
-int symmetrize_lower(int n, const double *A, long lda, double *F, long ldf, cudaStream_t s)
-{
-    dim3 g((unsigned)((n + 31) / 32), (unsigned)((n + 31) / 32)), blk(32, 8);
-    symmetrize_lower_kernel<<<g, blk, 0, s>>>(n, A, lda, F, ldf);
-    return cuda_fail(cudaGetLastError(), "symmetrize");
-}
-
 // F (n*n doubles of workspace) <- the lower triangle of A mirrored: call before
 // the eigensolver overwrites A.
 int refine_prepare(int n, const double *A, long lda, double *F, cudaStream_t s)

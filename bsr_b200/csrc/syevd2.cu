@@ -107,35 +107,113 @@ __global__ void __launch_bounds__(Q1H) q1_tmerge_kernel(const double *__restrict
 
 namespace bsrg {
 
-int symmetrize_lower(int n, const double *A, long lda, double *F, long ldf, cudaStream_t s);   // refine.cu
 
 // Workspace of dense_syevd in doubles (everything but the output Z)
+// ---------------------------------------------------------------------------
+// the working copy, its scale, and what a non-finite entry gives
+// ---------------------------------------------------------------------------
+// The sums of squares of the reductions hold for entries of 2^-300 .. 2^300; a matrix outside is
+// solved scaled by a power of two (exact both ways), one with a NaN or an infinity as zeros with NaN
+// results, so that no later kernel meets one.  One more pass over the triangle: 9 us at n = 2176, 53 at 7810.
+constexpr unsigned long long kInfBits = 0x7ff0000000000000ull;
+
+// max |A(i,j)|, i >= j, as bits (which order as the values do; a NaN is above infinity)
+__global__ void __launch_bounds__(256) amax_kernel(int n, const double *__restrict__ A, long lda,
+                                                   unsigned long long *amax)
+{
+    unsigned long long m = 0;
+    for (int j = blockIdx.x; j < n; j += gridDim.x) {
+        const double *col = A + (long)lda * j;
+        for (int i = j + threadIdx.x; i < n; i += 256)
+            m = max(m, (unsigned long long)__double_as_longlong(col[i]) & 0x7fffffffffffffffull);
+    }
+    for (int o = 16; o > 0; o >>= 1) m = max(m, __shfl_xor_sync(0xffffffffu, m, o));
+    if ((threadIdx.x & 31) == 0 && m) atomicMax(amax, m);
+}
+
+// the exponent of the power of two that the matrix is divided by
+__device__ __forceinline__ int scale_exp(unsigned long long bits)
+{
+    if (bits == 0 || bits >= kInfBits) return 0;
+    int q;
+    frexp(__longlong_as_double((long long)bits), &q);
+    return q < -300 || q > 300 ? q : 0;
+}
+
+// F = the symmetric matrix of A's lower triangle, scaled; 32 x 32 tiles
+__global__ void __launch_bounds__(256) work_copy_kernel(int n, const double *__restrict__ A, long lda,
+                                                        double *__restrict__ F, const unsigned long long *amax)
+{
+    __shared__ double tile[32][33];
+    const int bi = blockIdx.x, bj = blockIdx.y, tx = threadIdx.x, ty = threadIdx.y;
+    if (bi < bj) return;
+    const bool bad = *amax >= kInfBits;
+    const int q2 = scale_exp(*amax);
+    for (int q = ty; q < 32; q += 8) {
+        const int i = bi * 32 + tx, j = bj * 32 + q;
+        double v = 0.0;
+        if (i < n && j < n && !bad) v = i >= j ? A[i + (long)lda * j] : A[j + (long)lda * i];
+        if (q2) v = scalbn(v, -q2);
+        tile[q][tx] = v;
+        if (i < n && j < n) F[i + (long)n * j] = v;
+    }
+    __syncthreads();
+    if (bi == bj) return;
+    for (int q = ty; q < 32; q += 8) {
+        const int i = bj * 32 + tx, j = bi * 32 + q;
+        if (i < n && j < n) F[i + (long)n * j] = tile[tx][q];
+    }
+}
+
+// x (nx values) and y (ny) back to the matrix's scale; for a non-finite matrix these and Z are NaN
+__global__ void __launch_bounds__(256) work_finish_kernel(long nx, double *x, long ny, double *y, int n, double *Z,
+                                                          long ldz, const unsigned long long *amax)
+{
+    const bool bad = *amax >= kInfBits;
+    const int q2 = scale_exp(*amax);
+    if (!bad && q2 == 0) return;
+    const long t0 = blockIdx.x * 256L + threadIdx.x, step = gridDim.x * 256L;
+    for (long i = t0; i < nx; i += step) x[i] = bad ? NAN : scalbn(x[i], q2);
+    for (long i = t0; i < ny; i += step) y[i] = bad ? NAN : scalbn(y[i], q2);
+    if (bad && Z)
+        for (long i = t0; i < (long)n * n; i += step) Z[i % n + ldz * (i / n)] = NAN;
+}
+
 // The workspace carve-up of syevd2_impl, as offsets (doubles, 32-aligned); the size
 // function and the solver use this one layout.
 struct Syevd2Layout {
     size_t Wk, AB, V1, T1, V2, tau2, Tq, dv, ev, VYV, X, T, Mp, part, gram, flags, W1, W2, Vg, Gq, Tg,
-        gemm_ws, dcw, total;
+        gemm_ws, gemm_doubles, dcw, total;
 };
 
-static Syevd2Layout syevd2_layout(int n)
+// vectors false: what the reduction and the eigenvalues need (no reflectors are kept)
+static Syevd2Layout syevd2_layout(int n, bool vectors)
 {
     Syevd2Layout L{};
     const size_t nn = (size_t)n * n;
     const size_t S = (size_t)sweep_steps(n, 0) + 1;
     size_t off = 0;
     auto take = [&](size_t cnt) { off = (off + 31) & ~(size_t)31; size_t p = off; off += cnt; return p; };
-    // the fragments of Q2 take the place of the reduction's working copy and of the divide and conquer's
-    // workspace, which are through by then
-    L.Wk = L.Tq = take(nn);
-    L.dcw = take(dc_workspace_bytes(n) / 8 + 8);
-    off = std::max(off, L.Tq + q2_fragment_doubles(n));
+    L.Wk = take(nn);
+    if (vectors) {
+        // the fragments of Q2 take the place of the reduction's working copy and of the divide and
+        // conquer's workspace, which are through by then
+        L.Tq = L.Wk;
+        L.dcw = take(dc_workspace_bytes(n) / 8 + 8);
+        off = std::max(off, L.Tq + q2_fragment_doubles(n));
+        L.V1 = take(sy2sb_vsave_doubles(n));
+        L.T1 = take((size_t)(sy2sb_panels(n) + 1) * NB * NB);
+        L.V2 = take((size_t)n * S * NB);
+        L.tau2 = take((size_t)n * S);
+        L.W1 = take((size_t)Q1W * n);
+        L.W2 = take(std::max((size_t)Q1W * n, (size_t)(Q1W / 2) * (Q1W / 2)));   // also the T merges' temporary
+        L.Vg = take((size_t)Q1W * n);
+        L.Gq = take((size_t)Q1W * Q1W);
+        L.Tg = take((size_t)Q1W * Q1W);
+    }
     L.AB = take((size_t)2 * LDAB * n);
-    L.V1 = take(sy2sb_vsave_doubles(n));
-    L.T1 = take((size_t)(sy2sb_panels(n) + 1) * NB * NB);
-    L.V2 = take((size_t)n * S * NB);
-    L.tau2 = take((size_t)n * S);
     L.dv = take(n);
-    L.ev = take(n + 1);
+    L.ev = take(n + 8);
     L.VYV = take((size_t)n * 6 * NB);               // two [V | Y | V] buffers
     L.X = take((size_t)n * NB);
     L.T = take(NB * NB);
@@ -143,35 +221,51 @@ static Syevd2Layout syevd2_layout(int n)
     L.part = take((size_t)(n / NB + 8) * 4 * NB);
     L.gram = take((size_t)(n / NB + 8) * NB * NB);
     L.flags = take(8);
-    L.W1 = take((size_t)Q1W * n);
-    L.W2 = take(std::max((size_t)Q1W * n, (size_t)(Q1W / 2) * (Q1W / 2)));   // also the T merges' temporary
-    L.Vg = take((size_t)Q1W * n);
-    L.Gq = take((size_t)Q1W * Q1W);
-    L.Tg = take((size_t)Q1W * Q1W);
-    L.gemm_ws = take(8 * (size_t)Q1W * n);
+    // split-K partials: of X (16 slices of n x NB), with vectors also of the group products
+    L.gemm_doubles = vectors ? 8 * (size_t)Q1W * n : 16 * (size_t)NB * n;
+    L.gemm_ws = take(L.gemm_doubles);
     L.total = off + 64;
     return L;
 }
 
-size_t syevd2_workspace_doubles(int n) { return syevd2_layout(n).total; }
+size_t syevd2_workspace_doubles(int n, bool vectors) { return syevd2_layout(n, vectors).total; }
+
+// wait for the stream; device-side waits that ran out report through flags[2], a non-finite matrix
+// gives *info = 1 (the results are NaN)
+static int syevd2_status(const char *who, const int *flags, int *info, cudaStream_t st)
+{
+    int h[10];
+    cudaError_t e;
+    if ((e = cudaMemcpyAsync(h, flags, sizeof(h), cudaMemcpyDeviceToHost, st)) != cudaSuccess ||
+        (e = cudaStreamSynchronize(st)) != cudaSuccess)
+        return cuda_fail(e, who);
+    if (h[2] != 0) {
+        set_error("%s: a device-side wait timed out (%s)", who,
+                  h[2] == 2 ? "bulge chasing" : h[2] == 3 ? "back-transformation wavefront" : "panel barrier");
+        return BSRG_ERR_CUDA;
+    }
+    if (info) *info = (((unsigned long long)(unsigned)h[9] << 32) | (unsigned)h[8]) >= kInfBits ? 1 : 0;
+    return BSRG_OK;
+}
 
 // Eigenvalues (ascending, w) and eigenvectors (Z, ldz) of the symmetric A (lower
 // triangle referenced).  Z may be A itself.  ws: syevd2_workspace_doubles(n).
 // tri_d / tri_e non-null: stop after the reduction and copy the tridiagonal (d: n, e: n-1) there
 static int syevd2_impl(bsrg_ctx *c, int n, const double *A, long lda, double *w, double *Z, long ldz, double *ws,
                        size_t ws_doubles, void *pinned, size_t pinned_bytes, int *launches, double *tri_d,
-                       double *tri_e)
+                       double *tri_e, int *info)
 {
     int nl = 0;
     if (n < 1) return BSRG_OK;
     cudaStream_t st = c->stream;
     cudaError_t e;
-    if (ws_doubles < syevd2_workspace_doubles(n)) { set_error("dsyevd: workspace too small"); return BSRG_ERR_NOMEM; }
+    const bool vectors = Z != nullptr;
+    if (ws_doubles < syevd2_workspace_doubles(n, vectors)) { set_error("dsyevd: workspace too small"); return BSRG_ERR_NOMEM; }
     if (n > 10240) { set_error("dsyevd: n=%d above 10240", n); return BSRG_ERR_ARG; }
     const int S = sweep_steps(n, 0) + 1;
-    const Syevd2Layout L = syevd2_layout(n);
-    double *Wk = ws + L.Wk, *AB = ws + L.AB, *V1 = ws + L.V1, *T1 = ws + L.T1;
-    double *V2 = ws + L.V2, *tau2 = ws + L.tau2, *Tq = ws + L.Tq;
+    const Syevd2Layout L = syevd2_layout(n, vectors);
+    double *Wk = ws + L.Wk, *AB = ws + L.AB, *V1 = vectors ? ws + L.V1 : nullptr, *T1 = vectors ? ws + L.T1 : nullptr;
+    double *V2 = vectors ? ws + L.V2 : nullptr, *tau2 = ws + L.tau2, *Tq = ws + L.Tq;
     double *dv = ws + L.dv, *ev = ws + L.ev;
     Sy2sbWork sw;
     sw.VYV = ws + L.VYV;
@@ -184,16 +278,17 @@ static int syevd2_impl(bsrg_ctx *c, int n, const double *A, long lda, double *w,
     sw.Mp = ws + L.Mp;
     sw.part = ws + L.part;
     sw.gram = ws + L.gram;
-    int *flags = (int *)(ws + L.flags);            // bar[2], err, err2
+    int *flags = (int *)(ws + L.flags);            // bar[2], err, err2, ticket; from flags + 8: amax
+    unsigned long long *amax = (unsigned long long *)(flags + 8);
     sw.bar = (unsigned *)flags;
     sw.err = flags + 2;
     sw.ticket = (unsigned *)(flags + 4);
     double *W1 = ws + L.W1, *W2 = ws + L.W2;
     double *Vg = ws + L.Vg, *Gq = ws + L.Gq, *Tg = ws + L.Tg;
-    sw.gemm_ws_doubles = 8 * (size_t)Q1W * n;
+    sw.gemm_ws_doubles = L.gemm_doubles;
     sw.gemm_ws = ws + L.gemm_ws;
     double *dcw = ws + L.dcw;
-    if ((e = cudaMemsetAsync(flags, 0, 8 * sizeof(int), st)) != cudaSuccess)
+    if ((e = cudaMemsetAsync(flags, 0, 8 * sizeof(double), st)) != cudaSuccess)
         return cuda_fail(e, "dsyevd init");
     const int np = sy2sb_panels(n);
     double fl_band = 0.0, fl_chase = 0.0, fl_q2 = 0.0, fl_q1 = 0.0, fl_dc = 0.0;
@@ -205,7 +300,12 @@ static int syevd2_impl(bsrg_ctx *c, int n, const double *A, long lda, double *w,
     }
     // 1. full symmetric working copy, dense -> band
     stage_begin(c, 9);
-    int rc = symmetrize_lower(n, A, lda, Wk, n, st);
+    amax_kernel<<<(unsigned)std::min(n, 148 * 8), 256, 0, st>>>(n, A, lda, amax);
+    {
+        const unsigned nt = (unsigned)((n + 31) / 32);
+        work_copy_kernel<<<dim3(nt, nt), dim3(32, 8), 0, st>>>(n, A, lda, Wk, amax);
+    }
+    int rc = cuda_fail(cudaGetLastError(), "dsyevd working copy");
     if (rc == BSRG_OK) rc = sy2sb(st, n, Wk, n, V1, T1, sw);
     if (rc != BSRG_OK) return rc;
     rc = band_extract(n, Wk, n, AB, st);
@@ -221,19 +321,24 @@ static int syevd2_impl(bsrg_ctx *c, int n, const double *A, long lda, double *w,
     fl_chase = 4.0 * NB * (3.0 * NB) * (double)n * n / (2.0 * NB);      // whole windows, n^2 / (2 NB) steps
     stage_end(c, 10, 2);
     c->stage_flops[10] += fl_chase;
-    if (tri_d) {
-        int hf = 0;
-        if ((e = cudaMemcpyAsync(tri_d, dv, sizeof(double) * n, cudaMemcpyDeviceToDevice, st)) != cudaSuccess ||
-            (n > 1 && (e = cudaMemcpyAsync(tri_e, ev, sizeof(double) * (n - 1), cudaMemcpyDeviceToDevice, st)) !=
-                          cudaSuccess) ||
-            (e = cudaMemcpyAsync(&hf, flags + 2, sizeof(int), cudaMemcpyDeviceToHost, st)) != cudaSuccess ||
-            (e = cudaStreamSynchronize(st)) != cudaSuccess)
-            return cuda_fail(e, "dsytrd_2stage");
-        if (hf != 0) {
-            set_error("dsytrd_2stage: a device-side wait timed out (%s)", hf == 2 ? "bulge chasing" : "panel barrier");
-            return BSRG_ERR_CUDA;
+    if (!vectors) {
+        // the tridiagonal, or its eigenvalues
+        if (tri_d) {
+            if ((e = cudaMemcpyAsync(tri_d, dv, sizeof(double) * n, cudaMemcpyDeviceToDevice, st)) != cudaSuccess ||
+                (n > 1 && (e = cudaMemcpyAsync(tri_e, ev, sizeof(double) * (n - 1), cudaMemcpyDeviceToDevice, st)) !=
+                              cudaSuccess))
+                return cuda_fail(e, "dsytrd_2stage");
+            work_finish_kernel<<<8, 256, 0, st>>>(n, tri_d, n - 1, tri_e, n, nullptr, 0, amax);
+        } else {
+            stage_begin(c, 11);
+            rc = tridiag_values(st, n, dv, ev, w, ev + n);
+            stage_end(c, 11, 3);
+            if (rc != BSRG_OK) return rc;
+            work_finish_kernel<<<8, 256, 0, st>>>(n, w, 0, nullptr, n, nullptr, 0, amax);
+            c->stage_flops[6] += fl_band + fl_chase;
+            if (launches) *launches = 3 + np * 6 + 6;
         }
-        return BSRG_OK;
+        return syevd2_status(tri_d ? "dsytrd_2stage" : "dsyevd", flags, info, st);
     }
     // 3. tridiagonal eigenpairs into Z
     stage_begin(c, 11);
@@ -297,29 +402,23 @@ static int syevd2_impl(bsrg_ctx *c, int n, const double *A, long lda, double *w,
     }
     stage_end(c, 13, 10 * ((np + Q1_GROUP - 1) / Q1_GROUP));
     c->stage_flops[13] += fl_q1;
-    // device-side waits report through the flags
-    int hflag[2] = {0, 0};
-    if ((e = cudaMemcpyAsync(hflag, flags + 2, sizeof(int) * 2, cudaMemcpyDeviceToHost, st)) != cudaSuccess ||
-        (e = cudaStreamSynchronize(st)) != cudaSuccess)
-        return cuda_fail(e, "dsyevd");
+    work_finish_kernel<<<148, 256, 0, st>>>(n, w, 0, nullptr, n, Z, ldz, amax);
+    rc = syevd2_status("dsyevd", flags, info, st);
+    if (rc != BSRG_OK) return rc;
     fl_dc = dc_gemm_flops(n, pinned, nmerge);
     c->stage_flops[11] += fl_dc;
     c->stage_flops[6] += fl_band + fl_chase + fl_dc + fl_q2 + fl_q1;
-    if (hflag[0] != 0) {
-        set_error("dsyevd: a device-side wait timed out (%s)",
-                  hflag[0] == 2 ? "bulge chasing" : hflag[0] == 3 ? "back-transformation wavefront" : "panel barrier");
-        return BSRG_ERR_CUDA;
-    }
     // kernels of this library per call
-    nl = 2 + np * 6 + 2 + ndc + (n > 2 ? 2 : 0) + 3 * np;
+    nl = 4 + np * 6 + 2 + ndc + (n > 2 ? 2 : 0) + 3 * np;
     if (launches) *launches = nl;
     return BSRG_OK;
 }
 
 int dense_syevd(bsrg_ctx *c, int n, const double *A, long lda, double *w, double *Z, long ldz, double *ws,
-                size_t ws_doubles, void *pinned, size_t pinned_bytes, int *launches)
+                size_t ws_doubles, void *pinned, size_t pinned_bytes, int *launches, int *info)
 {
-    return syevd2_impl(c, n, A, lda, w, Z, ldz, ws, ws_doubles, pinned, pinned_bytes, launches, nullptr, nullptr);
+    return syevd2_impl(c, n, A, lda, w, Z, ldz, ws, ws_doubles, pinned, pinned_bytes, launches, nullptr, nullptr,
+                       info);
 }
 
 }  // namespace bsrg
@@ -332,10 +431,10 @@ extern "C" int bsrg_dsytrd_2stage(bsrg_ctx *c, int n, const double *A, int lda, 
     if (n < 0 || lda < (n > 0 ? n : 1)) { set_error("dsytrd_2stage: n=%d lda=%d", n, lda); return BSRG_ERR_ARG; }
     if (n == 0) return BSRG_OK;
     cudaSetDevice(c->device);
-    int rc = ctx_reserve(c, syevd2_workspace_doubles(n) * sizeof(double) + 1024);
+    int rc = ctx_reserve(c, syevd2_workspace_doubles(n, false) * sizeof(double) + 1024);
     if (rc != BSRG_OK) return rc;
     rc = syevd2_impl(c, n, A, lda, nullptr, nullptr, n, (double *)c->ws, c->ws_bytes / sizeof(double), nullptr, 0,
-                     nullptr, d, e);
+                     nullptr, d, e, nullptr);
     cudaEventRecord(c->ev_stage, c->stream);
     return rc;
 }
@@ -355,7 +454,7 @@ extern "C" int bsrg_dsyevd(bsrg_ctx *c, int n, const double *A, int lda, double 
     cudaError_t e = cudaEventSynchronize(c->ev_stage);     // the staging's last copies are through
     if (e != cudaSuccess) return cuda_fail(e, "dsyevd staging");
     rc = dense_syevd(c, n, A, lda, w, Z, ldz, (double *)c->ws, c->ws_bytes / sizeof(double), c->pinned,
-                     c->pinned_bytes, nullptr);
+                     c->pinned_bytes, nullptr, nullptr);
     cudaEventRecord(c->ev_stage, c->stream);
     return rc;
 }

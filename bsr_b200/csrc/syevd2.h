@@ -19,7 +19,8 @@ __device__ __forceinline__ unsigned long long gtime()
 __host__ __device__ __forceinline__ int sweep_steps(int n, int j) { return j <= n - 3 ? (n - 3 - j) / NB + 1 : 0; }
 
 // stage 1 (band_reduce.cu): the lower triangle of A to a band of width NB in place.  The panels' V go to
-// Vsave one after another (panel p: m_p x NB, m_p = n - (p + 1) NB, ld m_p), their T to Tsave + p NB^2.
+// Vsave one after another (panel p: m_p x NB, m_p = n - (p + 1) NB, ld m_p), their T to Tsave + p NB^2 (both null:
+// not kept).
 struct Sy2sbWork {
     double *VYV;       // m x 3NB
     double *VYV2;      // the second [V | Y | V] buffer (panels alternate while the look-ahead runs)
@@ -43,7 +44,7 @@ int sy2sb(cudaStream_t st, int n, double *A, long lda, double *Vsave, double *Ts
 
 // stage 2 (bulge.cu).  band_extract: the band of A (its NB subdiagonals) into AB, 2 LDAB n doubles;
 // bulge_chase: AB to tridiagonal form, d (n) and e (n-1), one cooperative kernel.  Reflector i of
-// sweep j goes to V2[((long)j S + i) NB ..] and tau2[(long)j S + i].  *err (zero on entry) is set to
+// sweep j goes to V2[((long)j S + i) NB ..] and tau2[(long)j S + i] unless V2 is null.  *err (zero on entry) is set to
 // 2 if a wait runs out.
 int band_extract(int n, const double *A, long lda, double *AB, cudaStream_t s);
 int bulge_chase(int n, double *AB, double *d, double *e, double *V2, double *tau2, int S, int *err, int nsm,

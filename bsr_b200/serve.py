@@ -31,7 +31,7 @@ from . import shard
 
 class Request:
     __slots__ = ("rid", "sym", "want_vectors", "t_submit", "t_start", "t_done", "result", "error", "event", "nbytes",
-                 "barrier")
+                 "barrier", "eigensolver")
 
     def __init__(self, rid, sym, want_vectors):
         self.rid, self.sym, self.want_vectors = rid, sym, want_vectors
@@ -39,6 +39,7 @@ class Request:
         self.result = self.error = None
         self.event = threading.Event()
         self.nbytes = 0
+        self.eigensolver = "auto"
         self.barrier = None       # warm-up requests: the worker waits here after releasing it
 
     def wait(self, timeout=None):
@@ -53,7 +54,7 @@ class Request:
         return None if self.t_done is None else self.t_done - self.t_submit
 
 
-OWN_EIG_MIN = 7000      # diag_hd's default crossover to the library's dense eigensolver (rows)
+OWN_EIG_MIN = 640       # diag_hd's default crossover to the library's dense eigensolver (rows, with vectors)
 
 
 def request_bytes(nch, ns, lch, ks, want_vectors=True, own_eig=False, mixed=False):
@@ -169,10 +170,16 @@ class PartialWaveServer:
         khm = shard.symmetry_dims(sym["nch"], self.ns, sym["lch"], self.ks)[0]
         own = self.eigensolver == "own" or (self.eigensolver == "auto" and khm >= OWN_EIG_MIN)
         nb = request_bytes(sym["nch"], self.ns, sym["lch"], self.ks, want_vectors, own_eig=own, mixed=self.mixed)
+        eig = self.eigensolver
+        if eig == "auto" and nb > self.budget:
+            # the library's eigensolver needs more workspace than cuSOLVER's
+            eig = "lib"
+            nb = request_bytes(sym["nch"], self.ns, sym["lch"], self.ks, want_vectors, mixed=self.mixed)
         with self._lock:
             r = Request(self._next_id, sym, want_vectors)
             self._next_id += 1
         r.nbytes = nb
+        r.eigensolver = eig
         r.t_submit = time.perf_counter()
         if nb > self.budget:
             r.error = "request needs %.2f GB, above the HBM budget of %.2f GB" % (nb / 1e9, self.budget / 1e9)
@@ -229,7 +236,6 @@ class PartialWaveServer:
         with torch.cuda.stream(stream):
             ctx = core.Context(stream=stream)
             ctx.use_tables(self.tables)
-            ctx.set_eigensolver(self.eigensolver)
             ctx.set_precision(self.mixed)
             while True:
                 r = self.queue.take()
@@ -238,6 +244,7 @@ class PartialWaveServer:
                 r.t_start = time.perf_counter()
                 try:
                     s = r.sym
+                    ctx.set_eigensolver(r.eigensolver)
                     H = core.assemble(ctx, self.basis, self.z, s["lch"], s["ech"], self.P, self.kmax, s["coefs"])
                     res = core.diag_hd(ctx, self.basis, s["lch"], H["hcc"], want_vectors=r.want_vectors)
                     ev = res["eval"].cpu().numpy()          # synchronises this worker's stream

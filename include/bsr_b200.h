@@ -328,10 +328,11 @@ int bsrg_ctx_set_refine(bsrg_ctx *c, int on);
 int bsrg_ctx_set_precision(bsrg_ctx *c, int mixed);
 /* ---- No counterpart in the reference (its DSYEV call is diag_hd.f90:312):
  *      which dense eigensolver bsrg_diag_hd uses on this context.  which = 0
- *      (default): the library's two-stage solver from 7000 rows of the dense
- *      problem (where it was measured faster than cuSOLVER's syevd on a B200)
- *      and cuSOLVER's below; 1: the library's at every size up to 10240 rows;
- *      2: cuSOLVER's at every size.  Contexts that solve concurrently on
+ *      (default): the library's two-stage solver from 640 rows of the dense
+ *      problem, 256 without eigenvectors (where it was measured faster than
+ *      cuSOLVER's syevd on a B200), up to 10240 rows and while its workspace
+ *      fits the device, and cuSOLVER's otherwise; 1: the library's at every
+ *      size up to 10240 rows; 2: cuSOLVER's at every size.  Contexts that solve concurrently on
  *      several streams do better with 1: the library's solver leaves most of
  *      the GPU to the other streams where cuSOLVER's reduction serialises
  *      them.  The environment variable BSRG_EIG=own|lib overrides it. */
