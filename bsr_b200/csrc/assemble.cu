@@ -1040,6 +1040,15 @@ __global__ void acf_kernel(int ns, int ks, int nch, int k, int ng, const GroupDe
 // ---------------------------------------------------------------------------
 // workspace helpers
 // ---------------------------------------------------------------------------
+cudaError_t ctx_read(bsrg_ctx *c, void *dst, const void *src, size_t bytes)
+{
+    void *to = c->back && bytes <= CTX_BACK ? c->back : dst;
+    cudaError_t e = cudaMemcpyAsync(to, src, bytes, cudaMemcpyDeviceToHost, c->stream);
+    if (e == cudaSuccess) e = cudaStreamSynchronize(c->stream);
+    if (e == cudaSuccess && to != dst) std::memcpy(dst, to, bytes);
+    return e;
+}
+
 int ctx_reserve(bsrg_ctx *c, size_t bytes)
 {
     if (c->ws_bytes >= bytes) return BSRG_OK;
@@ -1186,6 +1195,10 @@ int bsrg_ctx_create(int device, void *stream, bsrg_ctx **out)
         cudaGetLastError();
         c->aux_stream = nullptr;              // the band reduction then runs on one stream
     }
+    if (cudaMallocHost(&c->back, CTX_BACK) != cudaSuccess) {
+        cudaGetLastError();
+        c->back = nullptr;
+    }
     c->events = new std::vector<bsrg_stage_event>();
     c->pool = new std::vector<cudaEvent_t>();
     c->last_ipsol = new std::vector<int>();
@@ -1201,6 +1214,7 @@ int bsrg_ctx_destroy(bsrg_ctx *c)
     cudaStreamSynchronize(c->stream);
     if (c->ws) cudaFree(c->ws);
     if (c->pinned) cudaFreeHost(c->pinned);
+    if (c->back) cudaFreeHost(c->back);
     cudaEventDestroy(c->ev_stage);
     if (c->aux_stream) {
         cudaStreamSynchronize(c->aux_stream);
@@ -1549,8 +1563,7 @@ static int assemble_impl(bsrg_ctx *c, const bsrg_basis *b, double z, int nch, co
     if (mixed && d_tcerr) {
         // the tensor-core product reports a device-side wait that ran out through this flag
         int hf = 0;
-        cudaError_t em = cudaMemcpyAsync(&hf, d_tcerr, sizeof(int), cudaMemcpyDeviceToHost, s);
-        if (em == cudaSuccess) em = cudaStreamSynchronize(s);
+        const cudaError_t em = ctx_read(c, &hf, d_tcerr, sizeof(int));
         if (em != cudaSuccess) return cuda_fail(em, "assemble: mixed flag");
         if (hf == 2) { set_error("assemble: non-finite value in the direct contraction"); return BSRG_ERR_ARG; }
         if (hf) { set_error("assemble: a tensor-core wait timed out"); return BSRG_ERR_CUDA; }

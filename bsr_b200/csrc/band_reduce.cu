@@ -5,6 +5,8 @@
 // updated first and the next panel is factorised on a second stream beside the rest of the update.
 #include <algorithm>
 #include <cmath>
+#include <map>
+#include <mutex>
 
 #include <cooperative_groups.h>
 
@@ -600,6 +602,44 @@ size_t sy2sb_vsave_doubles(int n)
     return t + 64;
 }
 
+// Can the device hold the cluster form of the panel factorisation (16 CTAs with their shared memory)?  Asked
+// once per device: the two calls wait until other threads' copies to pageable memory are done.
+static cudaError_t panel_cluster_fits(bool *ok)
+{
+    static std::mutex mu;
+    static std::map<int, bool> fits;
+    int dev = 0;
+    cudaError_t e = cudaGetDevice(&dev);
+    if (e != cudaSuccess) return e;
+    std::lock_guard<std::mutex> lock(mu);
+    const auto known = fits.find(dev);
+    if (known != fits.end()) {
+        *ok = known->second;
+        return cudaSuccess;
+    }
+    const size_t smem_c = panel_smem(PC_ROWS);
+    int nclusters = 0;
+    if (cudaFuncSetAttribute(panel_qr_cluster_kernel, cudaFuncAttributeNonPortableClusterSizeAllowed, 1) ==
+            cudaSuccess &&
+        smem_attr(panel_qr_cluster_kernel, smem_c) == cudaSuccess) {
+        cudaLaunchConfig_t cfg = {};
+        cfg.gridDim = dim3(PC_MAXG);
+        cfg.blockDim = dim3(PC_NT);
+        cfg.dynamicSmemBytes = smem_c;
+        cudaLaunchAttribute attr[1];
+        attr[0].id = cudaLaunchAttributeClusterDimension;
+        attr[0].val.clusterDim.x = PC_MAXG;
+        attr[0].val.clusterDim.y = 1;
+        attr[0].val.clusterDim.z = 1;
+        cfg.attrs = attr;
+        cfg.numAttrs = 1;
+        if (cudaOccupancyMaxActiveClusters(&nclusters, panel_qr_cluster_kernel, &cfg) != cudaSuccess) nclusters = 0;
+    }
+    cudaGetLastError();
+    *ok = fits[dev] = nclusters >= 1;
+    return cudaSuccess;
+}
+
 int sy2sb(cudaStream_t st, int n, double *A, long lda, double *Vsave, double *Tsave, const Sy2sbWork &w)
 {
     cudaError_t e;
@@ -608,34 +648,8 @@ int sy2sb(cudaStream_t st, int n, double *A, long lda, double *Vsave, double *Ts
         (e = smem_attr(ypass1_kernel, sizeof(YpassSmem))) != cudaSuccess ||
         (e = smem_attr(ypass2_kernel, sizeof(YpassSmem))) != cudaSuccess)
         return cuda_fail(e, "sy2sb smem");
-    // the cluster form of the panel factorisation when a 16-CTA cluster with its shared memory fits
-    bool use_cluster = true;
-    if (use_cluster) {
-        const size_t smem_c = panel_smem(PC_ROWS);
-        if (cudaFuncSetAttribute(panel_qr_cluster_kernel, cudaFuncAttributeNonPortableClusterSizeAllowed, 1) !=
-                cudaSuccess ||
-            smem_attr(panel_qr_cluster_kernel, smem_c) !=
-                cudaSuccess) {
-            use_cluster = false;
-        } else {
-            cudaLaunchConfig_t cfg = {};
-            cfg.gridDim = dim3(PC_MAXG);
-            cfg.blockDim = dim3(PC_NT);
-            cfg.dynamicSmemBytes = smem_c;
-            cudaLaunchAttribute attr[1];
-            attr[0].id = cudaLaunchAttributeClusterDimension;
-            attr[0].val.clusterDim.x = PC_MAXG;
-            attr[0].val.clusterDim.y = 1;
-            attr[0].val.clusterDim.z = 1;
-            cfg.attrs = attr;
-            cfg.numAttrs = 1;
-            int nclusters = 0;
-            if (cudaOccupancyMaxActiveClusters(&nclusters, panel_qr_cluster_kernel, &cfg) != cudaSuccess ||
-                nclusters < 1)
-                use_cluster = false;
-        }
-        cudaGetLastError();
-    }
+    bool use_cluster = false;
+    if ((e = panel_cluster_fits(&use_cluster)) != cudaSuccess) return cuda_fail(e, "sy2sb device");
     // factorise panel p (columns j = p NB ..) on stream sq; its V goes to the [V | Y | V] buffer of p's parity
     auto factor_panel = [&](int p, size_t voff, cudaStream_t sq) -> int {
         const int j = p * NB, m = n - j - NB;

@@ -36,6 +36,7 @@ struct BulgeArgs {
     double *V2, *tau2;
     int S;
     int *err;
+    unsigned *ticket;               // the next sweep
 };
 
 struct BulgeSmem {
@@ -47,7 +48,7 @@ struct BulgeSmem {
     double Bt[NB][LD];              // B_i H_i
     int bready[LB], dready[LDW];    // steps staged, per loading warp
     int vready, doneB, doneD;       // steps whose reflector is known, whose blocks are stored
-    int quit;
+    int quit, sweep;
 };
 
 __device__ __forceinline__ ulonglong2 ld_pair(const ulonglong2 *p)
@@ -147,6 +148,11 @@ __device__ __forceinline__ bool load_pairs(const ulonglong2 *p, const ulonglong2
 //   and load units is what the loading warps' looks and the updates share.
 // Measured (CUDA events) at n = 470, 1713, 4400, 7810: 3.0, 12.4, 33.1, 63.3 ms with the reflector,
 // the right update and the reductions on the chain and a flag per step; 1.5, 6.0, 15.8, 29.1 ms now.
+// Sweeps in flight from sweep j on: a sweep takes 2.0 us a step and follows its predecessor by 3.7 us.  More
+// CTAs than that would only look for work, and keep SMs from other streams (n = 4000: 14.6 ms with steps / 1.5
+// and steps / 2 CTAs, 14.9 ms with steps and steps / 2.5).
+__host__ __device__ inline int sweeps_in_flight(int n, int j) { return sweep_steps(n, j) / 2 + 4; }
+
 __global__ void __launch_bounds__(BULGE_NT, 1) bulge_kernel(BulgeArgs a)
 {
     extern __shared__ __align__(16) unsigned char bulge_sm[];
@@ -154,7 +160,16 @@ __global__ void __launch_bounds__(BULGE_NT, 1) bulge_kernel(BulgeArgs a)
     const int t = threadIdx.x & 31, w = threadIdx.x >> 5, n = a.n;
     ulonglong2 *AB = a.AB;
     auto at = [&](int r, int c) -> ulonglong2 * { return AB + (r - c) + (long)LDAB * c; };
-    for (int j = blockIdx.x; j < n - 2; j += gridDim.x) {
+    for (;;) {
+        // Sweeps are taken in order, so a sweep's predecessor is done or with a CTA that is running: no wait
+        // needs a CTA that is not.  The sweeps get shorter: a CTA that the rest cannot keep busy gives its SM back.
+        if (threadIdx.x == 0) {
+            const int next = (int)min(*(volatile unsigned *)a.ticket, (unsigned)n);
+            s.sweep = next >= n - 2 || (int)blockIdx.x >= sweeps_in_flight(n, next) ? n : (int)atomicAdd(a.ticket, 1u);
+        }
+        __syncthreads();
+        const int j = s.sweep;
+        if (j >= n - 2) return;
         const int nst = sweep_steps(n, j);
         const unsigned long long before = (unsigned long long)j, after = before + 1;
         if (threadIdx.x == 0) {
@@ -421,22 +436,18 @@ int band_extract(int n, const double *A, long lda, double *AB, cudaStream_t st)
     return cuda_fail(cudaGetLastError(), "dsyevd band");
 }
 
-int bulge_chase(int n, double *AB, double *d, double *e, double *V2, double *tau2, int S, int *err, int nsm,
-                cudaStream_t st)
+int bulge_chase(int n, double *AB, double *d, double *e, double *V2, double *tau2, int S, int *err, unsigned *ticket,
+                int nsm, cudaStream_t st)
 {
     cudaError_t rc;
     if (n > 2) {
         rc = smem_attr(bulge_kernel, sizeof(BulgeSmem));
         if (rc != cudaSuccess) return cuda_fail(rc, "dsyevd bulge chasing smem");
-        // Sweeps in flight: a sweep takes 2.0 us a step and follows its predecessor by 3.7 us.  More CTAs
-        // than that would only look for work, and keep SMs from other streams (n = 4000: 14.6 ms with
-        // steps / 1.5 and steps / 2 CTAs, 14.9 ms with steps and steps / 2.5).
-        const int want = (int)(sweep_steps(n, 0) / 2.0) + 4;
-        const int ctas = std::max(1, std::min(n - 2, std::min(nsm, want)));
-        BulgeArgs a{(ulonglong2 *)AB, n, V2, tau2, S, err};
-        void *args[] = {&a};
-        rc = cudaLaunchCooperativeKernel((const void *)bulge_kernel, ctas, BULGE_NT, args, sizeof(BulgeSmem), st);
-        if (rc != cudaSuccess) return cuda_fail(rc, "dsyevd bulge chasing");
+        // an ordinary launch: it starts with the SMs that other streams leave
+        const int ctas = std::max(1, std::min(n - 2, std::min(nsm, sweeps_in_flight(n, 0))));
+        BulgeArgs a{(ulonglong2 *)AB, n, V2, tau2, S, err, ticket};
+        bulge_kernel<<<ctas, BULGE_NT, sizeof(BulgeSmem), st>>>(a);
+        if ((rc = cudaGetLastError()) != cudaSuccess) return cuda_fail(rc, "dsyevd bulge chasing");
     }
     tridiag_extract_kernel<<<(n + 255) / 256, 256, 0, st>>>(n, (const ulonglong2 *)AB, d, e);
     return cuda_fail(cudaGetLastError(), "dsyevd tridiagonal");

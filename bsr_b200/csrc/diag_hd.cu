@@ -549,13 +549,12 @@ static int diag_hd_impl(bsrg_ctx *c, const bsrg_basis *b, int nch, const int *lc
         int rco = chan_own_solve(c, b, hcc, nch, npad, d_s0, d_nsol, AA, Wv, d_info, chan_ws, d_cflag);
         if (rco != BSRG_OK) { cusolverDnDestroyParams(params); return rco; }
         int hf[2] = {0, 0};
-        if ((e = cudaMemcpyAsync(hf, d_cflag, sizeof(hf), cudaMemcpyDeviceToHost, s)) != cudaSuccess ||
-            (e = cudaStreamSynchronize(s)) != cudaSuccess) {
+        if ((e = ctx_read(c, hf, d_cflag, sizeof(hf))) != cudaSuccess) {
             cusolverDnDestroyParams(params);
             return cuda_fail(e, "diag_hd channel solves");
         }
         own_done = hf[0] == 0 && hf[1] == 0;
-        chan_launches = 8;
+        chan_launches = 11;
         if (!own_done) c->chan_fallbacks++;
     }
     if (own_done) {
@@ -757,9 +756,7 @@ static int diag_hd_impl(bsrg_ctx *c, const bsrg_basis *b, int nch, const int *lc
         if (rr == BSRG_OK && oz_ws) {
             // the digit product reports a wait that ran out (1) or a non-finite input (2)
             int hf = 0;
-            if ((e = cudaMemcpyAsync(&hf, d_rflag + 1, sizeof(int), cudaMemcpyDeviceToHost, s)) != cudaSuccess ||
-                (e = cudaStreamSynchronize(s)) != cudaSuccess)
-                return cuda_fail(e, "diag_hd refine flag");
+            if ((e = ctx_read(c, &hf, d_rflag + 1, sizeof(int))) != cudaSuccess) return cuda_fail(e, "diag_hd refine flag");
             if (hf == 2) { set_error("diag_hd: non-finite value in the refinement product"); return BSRG_ERR_ARG; }
             if (hf) { set_error("diag_hd: a tensor-core wait timed out"); return BSRG_ERR_CUDA; }
         }

@@ -232,13 +232,11 @@ size_t syevd2_workspace_doubles(int n, bool vectors) { return syevd2_layout(n, v
 
 // wait for the stream; device-side waits that ran out report through flags[2], a non-finite matrix
 // gives *info = 1 (the results are NaN)
-static int syevd2_status(const char *who, const int *flags, int *info, cudaStream_t st)
+static int syevd2_status(bsrg_ctx *c, const char *who, const int *flags, int *info)
 {
     int h[10];
     cudaError_t e;
-    if ((e = cudaMemcpyAsync(h, flags, sizeof(h), cudaMemcpyDeviceToHost, st)) != cudaSuccess ||
-        (e = cudaStreamSynchronize(st)) != cudaSuccess)
-        return cuda_fail(e, who);
+    if ((e = ctx_read(c, h, flags, sizeof(h))) != cudaSuccess) return cuda_fail(e, who);
     if (h[2] != 0) {
         set_error("%s: a device-side wait timed out (%s)", who,
                   h[2] == 2 ? "bulge chasing" : h[2] == 3 ? "back-transformation wavefront" : "panel barrier");
@@ -278,7 +276,7 @@ static int syevd2_impl(bsrg_ctx *c, int n, const double *A, long lda, double *w,
     sw.Mp = ws + L.Mp;
     sw.part = ws + L.part;
     sw.gram = ws + L.gram;
-    int *flags = (int *)(ws + L.flags);            // bar[2], err, err2, ticket; from flags + 8: amax
+    int *flags = (int *)(ws + L.flags);            // bar[2], err, err2, two tickets; from flags + 8: amax
     unsigned long long *amax = (unsigned long long *)(flags + 8);
     sw.bar = (unsigned *)flags;
     sw.err = flags + 2;
@@ -316,7 +314,7 @@ static int syevd2_impl(bsrg_ctx *c, int n, const double *A, long lda, double *w,
     // 2. band -> tridiagonal
     int nsm = 148;
     cudaDeviceGetAttribute(&nsm, cudaDevAttrMultiProcessorCount, c->device);
-    rc = bulge_chase(n, AB, dv, ev, V2, tau2, S, sw.err, nsm, st);
+    rc = bulge_chase(n, AB, dv, ev, V2, tau2, S, sw.err, (unsigned *)(flags + 5), nsm, st);
     if (rc != BSRG_OK) return rc;
     fl_chase = 4.0 * NB * (3.0 * NB) * (double)n * n / (2.0 * NB);      // whole windows, n^2 / (2 NB) steps
     stage_end(c, 10, 2);
@@ -338,7 +336,7 @@ static int syevd2_impl(bsrg_ctx *c, int n, const double *A, long lda, double *w,
             c->stage_flops[6] += fl_band + fl_chase;
             if (launches) *launches = 3 + np * 6 + 6;
         }
-        return syevd2_status(tri_d ? "dsytrd_2stage" : "dsyevd", flags, info, st);
+        return syevd2_status(c, tri_d ? "dsytrd_2stage" : "dsyevd", flags, info);
     }
     // 3. tridiagonal eigenpairs into Z
     stage_begin(c, 11);
@@ -403,7 +401,7 @@ static int syevd2_impl(bsrg_ctx *c, int n, const double *A, long lda, double *w,
     stage_end(c, 13, 10 * ((np + Q1_GROUP - 1) / Q1_GROUP));
     c->stage_flops[13] += fl_q1;
     work_finish_kernel<<<148, 256, 0, st>>>(n, w, 0, nullptr, n, Z, ldz, amax);
-    rc = syevd2_status("dsyevd", flags, info, st);
+    rc = syevd2_status(c, "dsyevd", flags, info);
     if (rc != BSRG_OK) return rc;
     fl_dc = dc_gemm_flops(n, pinned, nmerge);
     c->stage_flops[11] += fl_dc;

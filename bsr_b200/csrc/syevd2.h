@@ -43,11 +43,11 @@ size_t sy2sb_vsave_doubles(int n);
 int sy2sb(cudaStream_t st, int n, double *A, long lda, double *Vsave, double *Tsave, const Sy2sbWork &w);
 
 // stage 2 (bulge.cu).  band_extract: the band of A (its NB subdiagonals) into AB, 2 LDAB n doubles;
-// bulge_chase: AB to tridiagonal form, d (n) and e (n-1), one cooperative kernel.  Reflector i of
+// bulge_chase: AB to tridiagonal form, d (n) and e (n-1), one kernel; ticket: zero.  Reflector i of
 // sweep j goes to V2[((long)j S + i) NB ..] and tau2[(long)j S + i] unless V2 is null.  *err (zero on entry) is set to
 // 2 if a wait runs out.
 int band_extract(int n, const double *A, long lda, double *AB, cudaStream_t s);
-int bulge_chase(int n, double *AB, double *d, double *e, double *V2, double *tau2, int S, int *err, int nsm,
+int bulge_chase(int n, double *AB, double *d, double *e, double *V2, double *tau2, int S, int *err, unsigned *ticket, int nsm,
                 cudaStream_t s);
 
 // back-transformation of stage 2 (q2_apply.cu): Z <- Q2 Z for the n columns of Z.  frag:
