@@ -186,6 +186,8 @@ struct Syevd2Layout {
         gemm_ws, gemm_doubles, dcw, total;
 };
 
+static int q1_groups(int n) { return (sy2sb_panels(n) + Q1_GROUP - 1) / Q1_GROUP; }
+
 // vectors false: what the reduction and the eigenvalues need (no reflectors are kept)
 static Syevd2Layout syevd2_layout(int n, bool vectors)
 {
@@ -209,7 +211,7 @@ static Syevd2Layout syevd2_layout(int n, bool vectors)
         L.W2 = take(std::max((size_t)Q1W * n, (size_t)(Q1W / 2) * (Q1W / 2)));   // also the T merges' temporary
         L.Vg = take((size_t)Q1W * n);
         L.Gq = take((size_t)Q1W * Q1W);
-        L.Tg = take((size_t)Q1W * Q1W);
+        L.Tg = take((size_t)q1_groups(n) * Q1W * Q1W);
     }
     L.AB = take((size_t)2 * LDAB * n);
     L.dv = take(n);
@@ -229,6 +231,61 @@ static Syevd2Layout syevd2_layout(int n, bool vectors)
 }
 
 size_t syevd2_workspace_doubles(int n, bool vectors) { return syevd2_layout(n, vectors).total; }
+
+// the panels of group gq, their V in V1
+static Q1Panels q1_panels(int n, int gq, const double *V1)
+{
+    Q1Panels P{};
+    const int np = sy2sb_panels(n);
+    size_t off = 0;
+    for (int p = 0; p < (gq + 1) * Q1_GROUP; p++) {
+        const int q = p - gq * Q1_GROUP, m = n - p * NB - NB;
+        if (q >= 0) {
+            P.V[q] = p < np ? V1 + off : nullptr;
+            P.m[q] = p < np ? m : 0;
+        }
+        if (p < np) off += (size_t)m * NB;
+    }
+    return P;
+}
+
+// T of every group's merged 256-column reflector: each 128-column half by pairwise merges of its panels' T
+// (q1_tmerge_kernel), then the off-diagonal block -T_a G_ab T_b by two GEMMs.  They need the reduction's V and T
+// only, and a CTA or a few each: on the second stream they pass beside the chase, which leaves SMs over
+// (the stage, n = 1713: 2.30 -> 0.71 ms, n = 7810: 40.3 -> 32.7; the chase takes as long as before).
+static int q1_tfactors(int n, const double *V1, const double *T1, double *Vg, double *Gq, double *W2, double *Tg,
+                       double *gemm_ws, size_t gemm_ws_doubles, cudaStream_t st)
+{
+    cudaError_t e;
+    const int ngrp = q1_groups(n);
+    if ((e = smem_attr(q1_tmerge_kernel, Q1M_SMEM)) != cudaSuccess) return cuda_fail(e, "dsyevd Q1 smem");
+    if ((e = cudaMemsetAsync(Tg, 0, sizeof(double) * Q1W * Q1W * ngrp, st)) != cudaSuccess)
+        return cuda_fail(e, "dsyevd Q1 T");
+    for (int gq = 0; gq < ngrp; gq++) {
+        const int p0 = gq * Q1_GROUP, m0 = n - p0 * NB - NB;
+        const Q1Panels P = q1_panels(n, gq, V1);
+        double *T = Tg + (size_t)gq * Q1W * Q1W;
+        q1_gather_kernel<<<(unsigned)(((long)m0 * Q1W + 255) / 256), 256, 0, st>>>(m0, P, Vg);
+        int rc = dgemm(true, false, Q1W, Q1W, m0, 1.0, Vg, m0, Vg, m0, 0.0, Gq, Q1W, st, gemm_ws, gemm_ws_doubles);
+        for (int hq = 0; hq < Q1_GROUP / 4 && rc == BSRG_OK; hq++) {
+            const long o = (long)hq * Q1H * (Q1W + 1);
+            q1_tmerge_kernel<<<1, Q1H, Q1M_SMEM, st>>>(Gq + o, P, 4 * hq, T1, p0, T + o);
+            rc = cuda_fail(cudaGetLastError(), "dsyevd Q1 T");
+        }
+        for (int w = Q1H; w < Q1W && rc == BSRG_OK; w *= 2)
+            for (int a0 = 0; a0 < Q1W && rc == BSRG_OK; a0 += 2 * w) {
+                const int b0 = a0 + w;
+                // Wq = G(a, b) T_b (w x w), then T(a, b) = -T_a Wq
+                rc = dgemm(false, false, w, w, w, 1.0, Gq + a0 + (long)Q1W * b0, Q1W, T + b0 + (long)Q1W * b0, Q1W,
+                           0.0, W2, w, st);
+                if (rc == BSRG_OK)
+                    rc = dgemm(false, false, w, w, w, -1.0, T + a0 + (long)Q1W * a0, Q1W, W2, w, 0.0,
+                               T + a0 + (long)Q1W * b0, Q1W, st);
+            }
+        if (rc != BSRG_OK) return rc;
+    }
+    return BSRG_OK;
+}
 
 // wait for the stream; device-side waits that ran out report through flags[2], a non-finite matrix
 // gives *info = 1 (the results are NaN)
@@ -310,6 +367,15 @@ static int syevd2_impl(bsrg_ctx *c, int n, const double *A, long lda, double *w,
     if (rc != BSRG_OK) return rc;
     stage_end(c, 9, 2 + np * 6);
     c->stage_flops[9] += fl_band;
+    if (vectors && np > 0) {
+        cudaStream_t sq = sw.aux ? sw.aux : st;
+        if (sw.aux && ((e = cudaEventRecord(sw.ev_y, st)) != cudaSuccess ||
+                       (e = cudaStreamWaitEvent(sw.aux, sw.ev_y, 0)) != cudaSuccess))
+            return cuda_fail(e, "dsyevd Q1 T");
+        rc = q1_tfactors(n, V1, T1, Vg, Gq, W2, Tg, sw.gemm_ws, sw.gemm_ws_doubles, sq);
+        if (rc != BSRG_OK) return rc;
+        if (sw.aux && (e = cudaEventRecord(sw.ev_c2, sw.aux)) != cudaSuccess) return cuda_fail(e, "dsyevd Q1 T");
+    }
     stage_begin(c, 10);
     // 2. band -> tridiagonal
     int nsm = 148;
@@ -352,53 +418,22 @@ static int syevd2_impl(bsrg_ctx *c, int n, const double *A, long lda, double *w,
     stage_end(c, 12, n > 2 ? 2 : 0);
     c->stage_flops[12] += fl_q2;
     stage_begin(c, 13);
+    if (sw.aux && np > 0 && (e = cudaStreamWaitEvent(st, sw.ev_c2, 0)) != cudaSuccess) return cuda_fail(e, "dsyevd Q1 T");
     {
-        std::vector<size_t> voff;
-        size_t vo = 0;
-        for (int j = 0; j + NB < n; j += NB) { voff.push_back(vo); vo += (size_t)(n - j - NB) * NB; }
-        const int ngrp = (np + Q1_GROUP - 1) / Q1_GROUP;
-        for (int gq = ngrp - 1; gq >= 0; gq--) {
+        for (int gq = q1_groups(n) - 1; gq >= 0; gq--) {
             const int p0 = gq * Q1_GROUP, r0 = p0 * NB + NB, m0 = n - r0;
-            Q1Panels P{};
-            for (int q = 0; q < Q1_GROUP; q++) {
-                const int p = p0 + q;
-                P.V[q] = p < np ? V1 + voff[p] : nullptr;
-                P.m[q] = p < np ? n - p * NB - NB : 0;
-            }
+            const Q1Panels P = q1_panels(n, gq, V1);
             q1_gather_kernel<<<(unsigned)(((long)m0 * Q1W + 255) / 256), 256, 0, st>>>(m0, P, Vg);
-            rc = dgemm(true, false, Q1W, Q1W, m0, 1.0, Vg, m0, Vg, m0, 0.0, Gq, Q1W, st, sw.gemm_ws,
-                       sw.gemm_ws_doubles);
-            if (rc != BSRG_OK) return rc;
-            // T of the merged 256-column reflector: each 128-column half by pairwise merges of its
-            // panels' T (q1_tmerge_kernel), then the off-diagonal block -T_a G_ab T_b by two GEMMs
-            if ((e = smem_attr(q1_tmerge_kernel, Q1M_SMEM)) != cudaSuccess)
-                return cuda_fail(e, "dsyevd Q1 smem");
-            if ((e = cudaMemsetAsync(Tg, 0, sizeof(double) * Q1W * Q1W, st)) != cudaSuccess)
-                return cuda_fail(e, "dsyevd Q1 T");
-            for (int hq = 0; hq < Q1_GROUP / 4; hq++) {
-                const long o = (long)hq * Q1H * (Q1W + 1);
-                q1_tmerge_kernel<<<1, Q1H, Q1M_SMEM, st>>>(Gq + o, P, 4 * hq, T1, p0, Tg + o);
-            }
-            for (int w = Q1H; w < Q1W; w *= 2)
-                for (int a0 = 0; a0 < Q1W; a0 += 2 * w) {
-                    const int b0 = a0 + w;
-                    // Wq = G(a, b) T_b (w x w), then T(a, b) = -T_a Wq
-                    rc = dgemm(false, false, w, w, w, 1.0, Gq + a0 + (long)Q1W * b0, Q1W, Tg + b0 + (long)Q1W * b0,
-                               Q1W, 0.0, W2, w, st);
-                    if (rc == BSRG_OK)
-                        rc = dgemm(false, false, w, w, w, -1.0, Tg + a0 + (long)Q1W * a0, Q1W, W2, w, 0.0,
-                                   Tg + a0 + (long)Q1W * b0, Q1W, st);
-                    if (rc != BSRG_OK) return rc;
-                }
+            const double *Tq1 = Tg + (size_t)gq * Q1W * Q1W;
             double *Zs = Z + r0;
             rc = dgemm(true, false, Q1W, n, m0, 1.0, Vg, m0, Zs, ldz, 0.0, W1, Q1W, st, sw.gemm_ws,
                        sw.gemm_ws_doubles);
-            if (rc == BSRG_OK) rc = dgemm(false, false, Q1W, n, Q1W, 1.0, Tg, Q1W, W1, Q1W, 0.0, W2, Q1W, st);
+            if (rc == BSRG_OK) rc = dgemm(false, false, Q1W, n, Q1W, 1.0, Tq1, Q1W, W1, Q1W, 0.0, W2, Q1W, st);
             if (rc == BSRG_OK) rc = dgemm(false, false, m0, n, Q1W, -1.0, Vg, m0, W2, Q1W, 1.0, Zs, ldz, st);
             if (rc != BSRG_OK) return rc;
         }
     }
-    stage_end(c, 13, 10 * ((np + Q1_GROUP - 1) / Q1_GROUP));
+    stage_end(c, 13, 10 * q1_groups(n));
     c->stage_flops[13] += fl_q1;
     work_finish_kernel<<<148, 256, 0, st>>>(n, w, 0, nullptr, n, Z, ldz, amax);
     rc = syevd2_status(c, "dsyevd", flags, info);
