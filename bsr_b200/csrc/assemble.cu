@@ -1073,11 +1073,12 @@ int ctx_reserve_pinned(bsrg_ctx *c, size_t bytes)
     cudaError_t e = cudaStreamSynchronize(c->stream);
     if (e != cudaSuccess) return cuda_fail(e, "pinned sync");
     if (c->pinned) cudaFreeHost(c->pinned);
-    c->pinned = nullptr;
+    c->pinned = c->back = nullptr;
     c->pinned_bytes = 0;
-    size_t want = bytes + (bytes >> 3);
-    e = cudaMallocHost(&c->pinned, want);
-    if (e != cudaSuccess) return cuda_fail(e, "pinned alloc");
+    const size_t want = (bytes + (bytes >> 3) + 15) & ~(size_t)15;
+    e = cudaMallocHost(&c->pinned, want + CTX_BACK);
+    if (e != cudaSuccess) { c->pinned = nullptr; return cuda_fail(e, "pinned alloc"); }
+    c->back = (char *)c->pinned + want;
     c->pinned_bytes = want;
     return BSRG_OK;
 }
@@ -1195,10 +1196,6 @@ int bsrg_ctx_create(int device, void *stream, bsrg_ctx **out)
         cudaGetLastError();
         c->aux_stream = nullptr;              // the band reduction then runs on one stream
     }
-    if (cudaMallocHost(&c->back, CTX_BACK) != cudaSuccess) {
-        cudaGetLastError();
-        c->back = nullptr;
-    }
     c->events = new std::vector<bsrg_stage_event>();
     c->pool = new std::vector<cudaEvent_t>();
     c->last_ipsol = new std::vector<int>();
@@ -1214,7 +1211,6 @@ int bsrg_ctx_destroy(bsrg_ctx *c)
     cudaStreamSynchronize(c->stream);
     if (c->ws) cudaFree(c->ws);
     if (c->pinned) cudaFreeHost(c->pinned);
-    if (c->back) cudaFreeHost(c->back);
     cudaEventDestroy(c->ev_stage);
     if (c->aux_stream) {
         cudaStreamSynchronize(c->aux_stream);

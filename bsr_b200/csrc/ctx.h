@@ -54,7 +54,7 @@ struct bsrg_ctx {
     int chan_fallbacks;                      // channel solves redone on the library path (orthogonality check)
     cudaStream_t aux_stream;                 // high-priority second stream (the band reduction's panels), or 0
     cudaEvent_t aux_ev[2];                   //   its hand-off events
-    void *back;                              // pinned, CTX_BACK bytes: what ctx_read reads back into
+    void *back;                              // the pinned buffer's last CTX_BACK bytes: ctx_read's
 };
 
 namespace bsrg {
@@ -74,7 +74,7 @@ struct Arena {
 
 // dst <- bytes (CTX_BACK at most) at src on the device, when the stream has come to them.  By way of pinned
 // memory: a copy to pageable memory waits inside the driver, where it holds up other threads' calls until this
-// stream is through (eight solves on four streams: 145 ms, and 112 ms by way of pinned memory).
+// stream is through (eight solves on four streams: 145 ms, and 116 ms by way of pinned memory).
 constexpr size_t CTX_BACK = 256;
 cudaError_t ctx_read(bsrg_ctx *c, void *dst, const void *src, size_t bytes);
 
