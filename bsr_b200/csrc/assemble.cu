@@ -1057,7 +1057,7 @@ int ctx_reserve(bsrg_ctx *c, size_t bytes)
     if (c->ws) cudaFree(c->ws);
     c->ws = nullptr;
     c->ws_bytes = 0;
-    size_t want = bytes + (bytes >> 3);
+    const size_t want = ctx_grown(bytes);
     e = cudaMalloc(&c->ws, want);
     if (e != cudaSuccess) return cuda_fail(e, "workspace alloc");
     c->ws_bytes = want;

@@ -28,6 +28,7 @@ void set_error(const char *fmt, ...)
 int cuda_fail(cudaError_t e, const char *where)
 {
     if (e == cudaSuccess) return BSRG_OK;
+    cudaGetLastError();          // reported here: the next launch's check must not find it (a failed allocation stays set)
     set_error("%s: %s", where, cudaGetErrorString(e));
     return e == cudaErrorMemoryAllocation ? BSRG_ERR_NOMEM : BSRG_ERR_CUDA;
 }

@@ -79,7 +79,8 @@ constexpr size_t CTX_BACK = 256;
 cudaError_t ctx_read(bsrg_ctx *c, void *dst, const void *src, size_t bytes);
 
 // make sure the context workspace holds at least `bytes`; synchronises the
-// stream before replacing a smaller buffer.
+// stream before replacing a smaller buffer by one of ctx_grown(bytes).
+inline size_t ctx_grown(size_t bytes) { return bytes + (bytes >> 3); }
 int ctx_reserve(bsrg_ctx *c, size_t bytes);
 int ctx_reserve_pinned(bsrg_ctx *c, size_t bytes);
 

@@ -484,8 +484,15 @@ static int diag_hd_impl(bsrg_ctx *c, const bsrg_basis *b, int nch, const int *lc
     }
     int rc = BSRG_OK;
     if (own_eig) {
-        rc = ctx_reserve(c, need + sizeof(double) * syevd2_workspace_doubles(khm_max, want_vectors) + 512);
-        if (rc != BSRG_OK && auto_eig) own_eig = false;
+        const size_t own_need = need + sizeof(double) * syevd2_workspace_doubles(khm_max, want_vectors) + 512;
+        // asked before the workspace that there is would be given up: a context on a full device solves on without
+        // a new allocation per call
+        size_t left = 0, total = 0;
+        if (auto_eig && c->ws_bytes < own_need && cudaMemGetInfo(&left, &total) == cudaSuccess &&
+            left + c->ws_bytes < ctx_grown(own_need))
+            own_eig = false;
+        if (own_eig) rc = ctx_reserve(c, own_need);
+        if (rc == BSRG_ERR_NOMEM && auto_eig) own_eig = false;
     }
     if (!own_eig) {
         if (!lib_sizes(khm_max)) {
