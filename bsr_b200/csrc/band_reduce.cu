@@ -105,9 +105,10 @@ __global__ void __launch_bounds__(PQ_NT) panel_qr_kernel(PanelArgs a)
         __syncthreads();
         if (tid == 0) {
             const double alpha = piv[c], sigma = tot[c];
-            if (sigma == 0.0) { sc_tau = 0.0; sc_scale = 0.0; sc_beta = alpha; }
+            const double nn = alpha * alpha + sigma;
+            if (sigma == 0.0 || nn < SMALL_SQ) { sc_tau = 0.0; sc_scale = 0.0; sc_beta = alpha; }
             else {
-                const double beta = -copysign(sqrt(alpha * alpha + sigma), alpha);
+                const double beta = -copysign(sqrt(nn), alpha);
                 sc_tau = (beta - alpha) / beta;
                 sc_scale = 1.0 / (alpha - beta);
                 sc_beta = beta;
@@ -298,9 +299,10 @@ __global__ void __launch_bounds__(PC_NT) panel_qr_cluster_kernel(PanelArgs a)
                 }
                 const double piv = buf[PC_MAXG][lane & 7];
                 const double sigma = __shfl_sync(0xffffffffu, tot, j), alpha = __shfl_sync(0xffffffffu, piv, j);
+                const double nn = alpha * alpha + sigma;
                 double tau = 0.0, scale = 0.0, beta = alpha;
-                if (sigma != 0.0) {
-                    beta = -copysign(sqrt(alpha * alpha + sigma), alpha);
+                if (sigma != 0.0 && nn >= SMALL_SQ) {
+                    beta = -copysign(sqrt(nn), alpha);
                     tau = (beta - alpha) / beta;
                     scale = 1.0 / (alpha - beta);
                 }

@@ -202,9 +202,9 @@ __global__ void __launch_bounds__(BULGE_NT, 1) bulge_kernel(BulgeArgs a)
                         g3 = fma(xv[c + 1].y, xv[c + 1].y, g3);
                     }
                     const double sig = (g0 + g1) + (g2 + g3), alpha = xv[0].x;
+                    const double nn = fma(alpha, alpha, sig);
                     double beta = alpha, binv = 0.0;
-                    if (sig != 0.0) {
-                        const double nn = fma(alpha, alpha, sig);
+                    if (sig != 0.0 && nn >= SMALL_SQ) {
                         binv = -copysign(rsqrt(nn), alpha);
                         beta = nn * binv;
                     }

@@ -112,9 +112,12 @@ namespace bsrg {
 // ---------------------------------------------------------------------------
 // the working copy, its scale, and what a non-finite entry gives
 // ---------------------------------------------------------------------------
-// The sums of squares of the reductions hold for entries of 2^-300 .. 2^300; a matrix outside is
-// solved scaled by a power of two (exact both ways), one with a NaN or an infinity as zeros with NaN
-// results, so that no later kernel meets one.  One more pass over the triangle: 9 us at n = 2176, 53 at 7810.
+// A matrix whose largest entry lies outside 2^-150 .. 2^150 is solved scaled by a power of two (exact both ways),
+// one with a NaN or an infinity as zeros with NaN results, so that no later kernel meets one.  Inside that range no
+// sum of squares overflows, nor does 2 / |u|^2 times an entry (bulge.cu) for any column whose sum of squares is
+// SMALL_SQ = 2^-700 at least.  Columns below that are dropped: their entries, under 2^-350, are less than 2^-199
+// of the largest, while a reflector made from squares near the smallest number would not be orthogonal.
+// One more pass over the triangle: 9 us at n = 2176, 53 at 7810.
 constexpr unsigned long long kInfBits = 0x7ff0000000000000ull;
 
 // max |A(i,j)|, i >= j, as bits (which order as the values do; a NaN is above infinity)
@@ -137,7 +140,7 @@ __device__ __forceinline__ int scale_exp(unsigned long long bits)
     if (bits == 0 || bits >= kInfBits) return 0;
     int q;
     frexp(__longlong_as_double((long long)bits), &q);
-    return q < -300 || q > 300 ? q : 0;
+    return q < -150 || q > 150 ? q : 0;
 }
 
 // F = the symmetric matrix of A's lower triangle, scaled; 32 x 32 tiles

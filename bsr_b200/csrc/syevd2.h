@@ -6,6 +6,8 @@ namespace bsrg {
 
 constexpr int NB = 32;              // bandwidth of the intermediate band matrix
 constexpr int LDAB = 2 * NB;        // rows of the band storage: the band and room for the bulges
+// A column whose sum of squares lies below this counts as zero in the reductions (see amax_kernel in syevd2.cu)
+constexpr double SMALL_SQ = 0x1p-700;
 constexpr unsigned long long WAIT_NS = 2000000000ull;   // bound of every device-side wait (2 s)
 
 __device__ __forceinline__ unsigned long long gtime()
