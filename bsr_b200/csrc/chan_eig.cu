@@ -236,6 +236,19 @@ chan_tridiag_kernel(int ns, int npad, const int *__restrict__ s0v, const int *__
 #pragma unroll
                 for (int q = 0; q < CH_Q; q++)
                     if (q == (k + 1) >> 5) alpha = __shfl_sync(0xffffffffu, x[q], (k + 1) & 31);
+                // squares near the smallest normal number have lost their bits: the column scaled by 2^500 (exact)
+                double down = 1.0;
+                if (fma(alpha, alpha, sigma) < 0x1p-900) {
+                    down = 0x1p-500;
+                    alpha *= 0x1p500;
+                    sigma = 0.0;
+#pragma unroll
+                    for (int q = 0; q < CH_Q; q++) {
+                        x[q] *= 0x1p500;
+                        if (32 * q + lane >= k + 2) sigma = fma(x[q], x[q], sigma);
+                    }
+                    sigma = warp_sum(sigma);
+                }
                 double beta, scal;
                 if (sigma == 0.0) {
                     last = 0.0; beta = alpha; scal = 0.0;
@@ -245,7 +258,7 @@ chan_tridiag_kernel(int ns, int npad, const int *__restrict__ s0v, const int *__
                     scal = 1.0 / (alpha - beta);
                 }
                 __syncwarp();
-                if (lane == 0) { egc[k] = beta; tgc[k] = last; }
+                if (lane == 0) { egc[k] = beta * down; tgc[k] = last; }
                 // the new reflector (1, x(k+2..) scal), also kept below its first entry for the back-transform
 #pragma unroll
                 for (int q = 0; q < CH_Q; q++) {
