@@ -173,6 +173,17 @@ __device__ __forceinline__ double blk_max(double v, double *sh)
     return r;
 }
 
+// min(1, max |T(i, j)|), what the deflation's tolerance scales the entries of z with
+__global__ void __launch_bounds__(1024) dc_norm_kernel(int n, const double *__restrict__ d, const double *__restrict__ e,
+                                                       double *norm)
+{
+    __shared__ double red[32];
+    double m = 0.0;
+    for (int i = threadIdx.x; i < n; i += blockDim.x) m = fmax(m, fmax(fabs(d[i]), i + 1 < n ? fabs(e[i]) : 0.0));
+    m = blk_max(m, red);
+    if (threadIdx.x == 0) *norm = fmin(1.0, m);
+}
+
 // exclusive sum over the block's threads; the total in *all
 __device__ __forceinline__ unsigned long long blk_scan(unsigned long long v, unsigned long long *sh,
                                                        unsigned long long *all)
@@ -196,7 +207,9 @@ __device__ __forceinline__ unsigned long long blk_scan(unsigned long long v, uns
 }
 
 // Sort, deflate and group one merge's columns (one CTA).  LAPACK's rules: an entry of z below the tolerance
-// deflates; of two neighbours among the others that are close, a rotation takes one out.  The rotations
+// deflates; of two neighbours among the others that are close, a rotation takes one out.  LAPACK's tolerance,
+// 8 eps max(|d|, |z|), is that of a T scaled to 1; T is not scaled here, so where it is smaller the entries of z,
+// which are not, count times its largest entry.  The rotations
 // are a chain (an entry that a rotation has changed meets the next one), so one thread walks them, but only
 // from the pairs that are close as they are: every thread has tested its pairs first.  The places of the
 // columns are prefix sums over the threads' stretches.  (One thread in all of it took 1.6 ms in five merge
@@ -207,7 +220,8 @@ __device__ __forceinline__ unsigned long long blk_scan(unsigned long long v, uns
 //   I: pos[K] Qg column of pole i | gsrc[k] child column of Qg column t | rot (pairs of Qg columns) ...
 __global__ void __launch_bounds__(512) dc_prep_kernel(const DcMerge *__restrict__ mg, const double *__restrict__ e,
                                                       const double *__restrict__ w, const double *__restrict__ Z,
-                                                      long ldz, double *ws, int *iws, int *scal)
+                                                      long ldz, double *ws, int *iws, int *scal,
+                                                      const double *__restrict__ norm)
 {
     extern __shared__ __align__(16) unsigned char dsm[];
     __shared__ double red[32];
@@ -259,7 +273,7 @@ __global__ void __launch_bounds__(512) dc_prep_kernel(const DcMerge *__restrict_
     md = blk_max(md, red);
     mz = blk_max(mz, red);
     const double rho = 2.0 * fabs(beta);
-    const double tol = 8.0 * 2.220446049250313e-16 * fmax(md, mz);
+    const double tol = 8.0 * 2.220446049250313e-16 * fmax(md, mz * *norm);
     const bool none = rho * mz <= tol;                      // all deflate
     // a thread's stretch of the sorted order
     const int per = (k + nt - 1) / nt, i0 = min(k, tid * per), i1 = min(k, i0 + per);
@@ -927,6 +941,8 @@ int tridiag_dc(cudaStream_t st, int n, double *d, const double *e, double *w, do
     DcMerge *h_mg = h.mg;
     for (size_t q = 0; q < splits.size(); q++) h_splits[q] = splits[q];
     for (size_t q = 0; q < leaves.size(); q++) { h_ls[q] = leaves[q].s; h_lk[q] = leaves[q].k1; }
+    double *norm = wsd + 2 * (size_t)n * n + 8 * (size_t)n;          // after the merges' vectors
+    dc_norm_kernel<<<1, 1024, 0, st>>>(n, d, e, norm);
     if (!splits.empty()) {
         if ((err = cudaMemcpyAsync(d_splits, h_splits, sizeof(int) * splits.size(), cudaMemcpyHostToDevice, st)) !=
             cudaSuccess)
@@ -969,7 +985,7 @@ int tridiag_dc(cudaStream_t st, int n, double *d, const double *e, double *w, do
         if ((err = smem_attr(dc_prep_kernel, smem_prep)) != cudaSuccess ||
             (err = smem_attr(dc_secular_kernel, smem_sec)) != cudaSuccess)
             return cuda_fail(err, "dstedc smem");
-        dc_prep_kernel<<<nm, 512, smem_prep, st>>>(mg, e, w, Z, ldz, wsd, wsi, sc);
+        dc_prep_kernel<<<nm, 512, smem_prep, st>>>(mg, e, w, Z, ldz, wsd, wsi, sc, norm);
         const dim3 gg((unsigned)((kmax + 127) / 128), (unsigned)((kmax + 31) / 32), nm);
         dc_gather_kernel<<<gg, 128, 0, st>>>(mg, Z, ldz, wsd, wsi);
         dc_rotate_kernel<<<dim3((unsigned)((kmax + 127) / 128), nm), 128, 0, st>>>(mg, sc, wsd, wsi);
@@ -992,7 +1008,7 @@ int tridiag_dc(cudaStream_t st, int n, double *d, const double *e, double *w, do
         if ((err = cudaMemcpyAsync(h_scal, d_scal, sizeof(int) * DC_NS * nmg, cudaMemcpyDeviceToHost, st)) != cudaSuccess)
             return cuda_fail(err, "dstedc counts");
     }
-    if (launches) *launches = nlaunch + 2;
+    if (launches) *launches = nlaunch + 3;
     return BSRG_OK;
 }
 
