@@ -25,6 +25,7 @@
 
 #include <cooperative_groups.h>
 
+#include "aux_join.h"
 #include "ctx.h"
 #include "dgemm.h"
 #include "syevd2.h"
@@ -331,6 +332,7 @@ static int syevd2_impl(bsrg_ctx *c, int n, const double *A, long lda, double *w,
     sw.aux = getenv("BSRG_NO_LOOKAHEAD") ? nullptr : c->aux_stream;
     sw.ev_y = c->aux_ev[0];
     sw.ev_c2 = c->aux_ev[1];
+    AuxJoin join(sw.aux, st, sw.ev_c2);
     sw.X = ws + L.X;
     sw.T = ws + L.T;
     sw.Mp = ws + L.Mp;
@@ -405,6 +407,7 @@ static int syevd2_impl(bsrg_ctx *c, int n, const double *A, long lda, double *w,
             c->stage_flops[6] += fl_band + fl_chase;
             if (launches) *launches = 3 + np * 6 + 6;
         }
+        join.done();                                // the reduction has joined the second stream
         return syevd2_status(c, tri_d ? "dsytrd_2stage" : "dsyevd", flags, info);
     }
     // 3. tridiagonal eigenpairs into Z
@@ -422,6 +425,7 @@ static int syevd2_impl(bsrg_ctx *c, int n, const double *A, long lda, double *w,
     c->stage_flops[12] += fl_q2;
     stage_begin(c, 13);
     if (sw.aux && np > 0 && (e = cudaStreamWaitEvent(st, sw.ev_c2, 0)) != cudaSuccess) return cuda_fail(e, "dsyevd Q1 T");
+    join.done();
     {
         for (int gq = q1_groups(n) - 1; gq >= 0; gq--) {
             const int p0 = gq * Q1_GROUP, r0 = p0 * NB + NB, m0 = n - r0;
