@@ -374,6 +374,12 @@ using namespace bsrg;
 // 21.5 / 26.1 at 1564, 51 / 81 at 3907, 126 / 380 at 7810)
 constexpr int kOwnEigMin = 640, kOwnValMin = 256;
 
+static int cholesky_failed(int pivot)
+{
+    set_error("BSR_HD: Cholesky factorization failed (overlap pivot %d)", pivot);
+    return BSRG_ERR_INFO;
+}
+
 // scc == NULL: the block-diagonal overlap (diag_ovl /= 0); otherwise the generalized
 // branch with the channel-channel overlap blocks of scc (diag_ovl = 0)
 static int diag_hd_impl(bsrg_ctx *c, const bsrg_basis *b, int nch, const int *lch, const double *hcc,
@@ -730,6 +736,12 @@ static int diag_hd_impl(bsrg_ctx *c, const bsrg_basis *b, int nch, const int *lc
                              (char *)c->pinned + o_dc_bytes, c->pinned_bytes - o_dc_bytes, &nlaunch, &eig_info);
         stage_end(c, 6, nlaunch);
         if (re != BSRG_OK) return re;
+        if (eig_info != 0 && gen) {
+            // a matrix reduced with a failed factor need not be finite: the factorisation's error comes first
+            int pivot = 0;
+            if ((e = ctx_read(c, &pivot, d_cinfo, sizeof(int))) != cudaSuccess) return cuda_fail(e, "diag_hd info");
+            if (pivot != 0) return cholesky_failed(pivot);
+        }
         if (eig_info != 0) { set_error("LAP_DSYEV: DSYEV(lapack) gives INFO = %d", eig_info); return BSRG_ERR_INFO; }
         if ((e = cudaMemsetAsync(d_info + nch, 0, sizeof(int), s)) != cudaSuccess) return cuda_fail(e, "diag_hd info");
     } else {
@@ -789,10 +801,7 @@ static int diag_hd_impl(bsrg_ctx *c, const bsrg_basis *b, int nch, const int *lc
     if (gen && (e = cudaMemcpyAsync(hi + o_fin + 1, d_cinfo, sizeof(int), cudaMemcpyDeviceToHost, s)) != cudaSuccess)
         return cuda_fail(e, "diag_hd info");
     if ((e = cudaStreamSynchronize(s)) != cudaSuccess) return cuda_fail(e, "diag_hd syevd");
-    if (gen && hi[o_fin + 1] != 0) {
-        set_error("BSR_HD: Cholesky factorization failed (overlap pivot %d)", hi[o_fin + 1]);
-        return BSRG_ERR_INFO;
-    }
+    if (gen && hi[o_fin + 1] != 0) return cholesky_failed(hi[o_fin + 1]);
     int hinfo = hi[o_fin];
     if (hinfo != 0) {
         set_error("LAP_DSYEV: DSYEV(lapack) gives INFO = %d", hinfo);
