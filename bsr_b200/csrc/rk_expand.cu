@@ -28,6 +28,8 @@
 // (NI = 1..4) and instruction fetches: 34 M instructions, 9.5 M of them adds and multiplies.  Two
 // chains per thread were no faster (72 us); three CTAs per SM beat two (70 us) and four (64 us).
 // Compiled with --fmad=false: the results equal the reference's order bit for bit.
+#include <algorithm>
+
 #include "bsrg_internal.h"
 
 namespace bsrg {
@@ -245,6 +247,7 @@ struct QArgs {
     double fine;
     const double *r1, *r2, *r3, *r4, *rkd;      // (ks*ks, nv) each; rkd (ks*ks, ks*ks, nv)
     double *rkb;
+    int z0;                                     // the launch's first pair of columns
 };
 
 // acc +- sum over the outer lo..hi-1 of x[outer] (row of inner terms y); the outer moments in registers,
@@ -347,7 +350,7 @@ __global__ void __launch_bounds__(32 * NWARP) qk_expand_kernel(QArgs a)
 {
     extern __shared__ double qsm[];                         // r1, r2, r3, r4 of the i pairs, then of the j pairs
     double (*I)[TQ * TI] = (double (*)[TQ * TI])qsm, (*J)[TQ * TJ] = (double (*)[TQ * TJ])(qsm + 4 * TQ * TI);
-    const int ip = blockIdx.z % a.ldp, jp = blockIdx.z / a.ldp, ks = a.ks;
+    const int z = a.z0 + (int)blockIdx.z, ip = z % a.ldp, jp = z / a.ldp, ks = a.ks;
     const bool band = blockIdx.y == 0;
     const int i0 = blockIdx.x * TI, j0 = band ? i0 - (ks - 1) : ((int)blockIdx.y - 1) * TJ;
     if (ip >= 2 * ks - 1 || jp >= 2 * ks - 1) {
@@ -425,11 +428,16 @@ int launch_mvk_cell(const bsrg_basis *b, const double *rkd1, const double *rkd2,
 int launch_mqk_cell(const bsrg_basis *b, const double *rkd1, const double *rkd2, const double *rkd3,
                     const double *rkd4, const double *rkd, double fine, double *rkb, int ldp, cudaStream_t s)
 {
-    const QArgs a{b->ks, b->ns, b->nv, ldp, fine, rkd1, rkd2, rkd3, rkd4, rkd, rkb};
+    QArgs a{b->ks, b->ns, b->nv, ldp, fine, rkd1, rkd2, rkd3, rkd4, rkd, rkb, 0};
     const int shm = 4 * TQ * (TI + TJ) * (int)sizeof(double);
     cudaError_t e = smem_attr(qk_expand_kernel, shm);
     if (e != cudaSuccess) return cuda_fail(e, "mqk_cell smem");
-    qk_expand_kernel<<<tiles(b, ldp), 32 * NWARP, shm, s>>>(a);
+    // a grid's z ends at 65535: more pairs of columns (ldp > 255) take more launches
+    dim3 grd = tiles(b, ldp);
+    for (const int pairs = (int)grd.z; a.z0 < pairs; a.z0 += 65535) {
+        grd.z = (unsigned)std::min(65535, pairs - a.z0);
+        qk_expand_kernel<<<grd, 32 * NWARP, shm, s>>>(a);
+    }
     return cuda_fail(cudaGetLastError(), "mqk_cell");
 }
 
