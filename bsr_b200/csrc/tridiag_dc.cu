@@ -942,8 +942,8 @@ int tridiag_dc(cudaStream_t st, int n, double *d, const double *e, double *w, do
     for (size_t q = 0; q < splits.size(); q++) h_splits[q] = splits[q];
     for (size_t q = 0; q < leaves.size(); q++) { h_ls[q] = leaves[q].s; h_lk[q] = leaves[q].k1; }
     double *norm = wsd + 2 * (size_t)n * n + 8 * (size_t)n;          // after the merges' vectors
-    dc_norm_kernel<<<1, 1024, 0, st>>>(n, d, e, norm);
     if (!splits.empty()) {
+        dc_norm_kernel<<<1, 1024, 0, st>>>(n, d, e, norm);
         if ((err = cudaMemcpyAsync(d_splits, h_splits, sizeof(int) * splits.size(), cudaMemcpyHostToDevice, st)) !=
             cudaSuccess)
             return cuda_fail(err, "dstedc upload");
@@ -1008,7 +1008,7 @@ int tridiag_dc(cudaStream_t st, int n, double *d, const double *e, double *w, do
         if ((err = cudaMemcpyAsync(h_scal, d_scal, sizeof(int) * DC_NS * nmg, cudaMemcpyDeviceToHost, st)) != cudaSuccess)
             return cuda_fail(err, "dstedc counts");
     }
-    if (launches) *launches = nlaunch + 3;
+    if (launches) *launches = nlaunch + (splits.empty() ? 1 : 3);
     return BSRG_OK;
 }
 
