@@ -125,20 +125,46 @@ __global__ void channel_weights_kernel(int nch, const int *__restrict__ ipsol, i
             if (rank == 0) isol[is] = i + 1;
         }
     }
-    if (__syncthreads_or(tie) && threadIdx.x == 0) {
-        for (int i = 0; i < nch; i++) ipt[i] = i;
+    if (__syncthreads_or(tie) && threadIdx.x < 32) {
+        // the exchange sort by one warp.  A pass takes the first largest weight on to place i1; every weight on the way
+        // that is larger than all before it passes its place to the one it beats (a NaN beats and is beaten by none).
+        const int lane = threadIdx.x;
+        for (int i = lane; i < nch; i += 32) ipt[i] = i;
+        __syncwarp();
         for (int i1 = 0; i1 < nch - 1; i1++) {
-            int j1 = ipt[i1];
-            for (int i2 = i1 + 1; i2 < nch; i2++) {
-                const int j2 = ipt[i2];
-                if (fabs(w[j1]) < fabs(w[j2])) {
-                    ipt[i2] = j1;
-                    j1 = j2;
+            double top = fabs(w[i1]);
+            int ch = ipt[i1];
+            for (int i0 = i1 + 1; i0 < nch; i0 += 32) {
+                const int i2 = i0 + lane;
+                const double x = i2 < nch ? fabs(w[i2]) : -1.0;
+                if (!__any_sync(0xffffffffu, top < x)) continue;
+                const int xc = i2 < nch ? ipt[i2] : 0;
+                double m = x >= 0.0 ? x : -1.0;              // the largest so far, in the chunk
+                for (int o = 1; o < 32; o <<= 1) {
+                    const double y = __shfl_up_sync(0xffffffffu, m, o);
+                    if (lane >= o) m = fmax(m, y);
                 }
+                m = __shfl_up_sync(0xffffffffu, m, 1);
+                const bool beats = top < x && (lane == 0 || m < x);
+                const unsigned all = __ballot_sync(0xffffffffu, beats), before = all & ((1u << lane) - 1);
+                const int from = before ? 31 - __clz(before) : 0, last = 31 - __clz(all);
+                const double pw = __shfl_sync(0xffffffffu, x, from);
+                const int pc = __shfl_sync(0xffffffffu, xc, from);
+                if (beats) {
+                    w[i2] = before ? pw : top;
+                    ipt[i2] = before ? pc : ch;
+                }
+                top = __shfl_sync(0xffffffffu, x, last);
+                ch = __shfl_sync(0xffffffffu, xc, last);
             }
-            ipt[i1] = j1;
+            __syncwarp();
+            if (lane == 0) {
+                w[i1] = top;
+                ipt[i1] = ch;
+            }
+            __syncwarp();
         }
-        isol[is] = ipt[0] + 1;
+        if (lane == 0) isol[is] = ipt[0] + 1;
     }
     if (iprm) {
         __syncthreads();
