@@ -50,7 +50,7 @@ def nvcc():
 def build(verbose=False, force=False):
     os.makedirs(BUILD, exist_ok=True)
     objs = []
-    headers = [os.path.join(CSRC, f) for f in os.listdir(CSRC) if f.endswith(".h")]
+    headers = [os.path.join(CSRC, f) for f in os.listdir(CSRC) if f.endswith((".h", ".cuh"))]
     headers.append(os.path.join(HERE, "..", "include", "bsr_b200.h"))
     hdr_mtime = max(os.path.getmtime(h) for h in headers)
     for unit, extra in UNITS.items():
