@@ -105,8 +105,8 @@ template <int TILE, bool KFAST, int NT> struct Stager {
     __device__ __forceinline__ void advance() { p += KFAST ? BK : BK * ld; }
 };
 
-// The same for a square symmetric A of which only the lower triangle is stored: element (m, k) is read
-// from (max, min), a tile wholly above the diagonal with the index order that keeps the reads coalesced.
+// The same for the diagonal tiles of a square symmetric A of which only the lower triangle is stored (tile_mma
+// takes the others as they are or transposed): element (m, k) is read from (max, min).
 template <int TILE, int NT> struct SymStager {
     static constexpr int N = TILE * BK / NT, LD = TILE + PAD;
     const double *base;
@@ -118,11 +118,10 @@ template <int TILE, int NT> struct SymStager {
     }
     __device__ __forceinline__ void part(double *s, int q, int krem) const
     {
-        const bool upper = t0 + TILE <= k0;
 #pragma unroll
         for (int i = 0; i < N / 4; i++) {
             const int idx = tid + (q * (N / 4) + i) * NT;
-            const int tl = upper ? idx / BK : idx % TILE, kl = upper ? idx % BK : idx / TILE;
+            const int tl = idx % TILE, kl = idx / TILE;
             const int gm = t0 + tl, gk = k0 + kl;
             const bool v = gm < size && kl < krem;
             cp_async8(s + kl * LD + tl, v ? (gm >= gk ? base + gm + (long)gk * ld : base + gk + (long)gm * ld) : base, v);
