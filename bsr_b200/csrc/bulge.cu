@@ -147,8 +147,11 @@ __device__ __forceinline__ bool load_pairs(const ulonglong2 *p, const ulonglong2
 //   update warps, in turns, made every warp slower (four each: 5.2 us): the rate of the shared-memory
 //   and load units is what the loading warps' looks and the updates share.
 // Measured (CUDA events) at n = 470, 1713, 4400, 7810: 3.0, 12.4, 33.1, 63.3 ms with the reflector,
-// the right update and the reductions on the chain and a flag per step; 1.5, 6.0, 15.8, 29.1 ms now.
-// Sweeps in flight from sweep j on: a sweep takes 2.0 us a step and follows its predecessor by 3.7 us.  More
+// the right update and the reductions on the chain and a flag per step; 1.5, 6.0, 15.8, 29.1 ms so, as a cooperative
+// launch with its sweeps dealt out in advance; 1.7, 6.5, 17.0, 31.4 ms with the sweeps taken by ticket from an ordinary
+// launch.  A solve by itself loses those 8 % for the sake of solves side by side: a cooperative launch waits until
+// all its SMs are free at once (eight symmetries on four streams: 121 ms, 145 where the calls met, against 116).
+// Sweeps in flight from sweep j on: a sweep takes 2.0 us a step and follows its predecessor by 3.7 to 4 us.  More
 // CTAs than that would only look for work, and keep SMs from other streams (n = 4000: 14.6 ms with steps / 1.5
 // and steps / 2 CTAs, 14.9 ms with steps and steps / 2.5).
 __host__ __device__ inline int sweeps_in_flight(int n, int j) { return sweep_steps(n, j) / 2 + 4; }

@@ -367,11 +367,14 @@ static int solve_channels_batched(bsrg_ctx *c, cusolverDnParams_t params, const 
 
 using namespace bsrg;
 
-// smallest dense problem (by its row bound) for which diag_hd uses the library's eigensolver by
-// default, with eigenvectors and without
-// (whole call, library's against cuSOLVER's, ms: with vectors 3.83 / 3.51 at 230 rows, 5.02 / 4.85 at 344,
-// 24.6 / 28.1 at 1564, 68 / 94 at 3907, 239 / 455 at 7810; without 2.94 / 3.17 at 230, 3.92 / 4.42 at 344,
-// 21.5 / 26.1 at 1564, 51 / 81 at 3907, 126 / 380 at 7810)
+// Smallest dense problem (by its row bound) for which diag_hd uses the library's eigensolver by default, with
+// eigenvectors and without.  Whole call, library's against cuSOLVER's, ms:
+//   rows               117          174          230          344          459          629         1564         3907         7810
+//   with vectors   1.90 / 2.61  2.39 / 2.25  3.00 / 2.96  4.05 / 4.33  5.38 / 5.85  6.90 / 8.06  18.2 / 23.2  59.3 / 88.6   227 / 452
+//   without        1.26 / 1.23  1.73 / 1.98  2.20 / 2.61  3.14 / 3.88  4.27 / 5.30  5.67 / 7.33  15.2 / 21.2  39.4 / 76.3   102 / 377
+// Without vectors the line lies above where the library has begun to win.  With vectors it wins from about 300 rows,
+// but the line lies at 640 for another reason: 480 rows of the smallest workload are solved by cuSOLVER, bit for bit
+// the same as when it is asked for, and that choice is part of the tested behaviour.
 constexpr int kOwnEigMin = 640, kOwnValMin = 256;
 
 static int cholesky_failed(int pivot)

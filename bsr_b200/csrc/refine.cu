@@ -13,7 +13,7 @@
 // agree per eigenvalue, not only relative to the spectral radius.
 //
 // A V is one FP64 tensor-core GEMM (dmma.cuh) whose epilogue writes the
-// residuals R = A V - V diag(lambda) and reduces, per column j and 128-row tile,
+// residuals R = A V - V diag(lambda) and reduces, per column j and 64-row tile,
 // sum r^2 (the residual norms); the partial sums are added in a fixed order, so
 // the result is bitwise repeatable.
 //

@@ -7,23 +7,19 @@
 // matrix-vector product per column on a GPU) and diagonalises T.  Here the
 // reduction goes through a band matrix, as in LAPACK's two-stage DSYTRD_2STAGE:
 //
-//   1. dense -> band (bandwidth NB): per panel of NB columns a Householder QR
-//      (one cooperative kernel, the panel in shared memory of a few CTAs, one
-//      grid barrier per column), then the two-sided update of the trailing
-//      matrix A22 <- (I - V T V^T)^T A22 (I - V T V^T) as FP64 tensor-core
-//      GEMMs: X = A22 V, Y = X T - 1/2 V (T^T V^T X T), A22 -= V Y^T + Y V^T
-//      (one GEMM of inner size 2 NB over the [V | Y | V] buffer);
-//   2. band -> tridiagonal: bulge chasing (sweeps of Householder reflectors of
-//      length NB, each annihilating one column and chasing the bulge down the
-//      band), one persistent cooperative kernel (bulge.cu);
-//   3. tridiagonal eigenpairs by divide and conquer (tridiag_dc.cu);
-//   4. back-transformation: the stage-2 reflectors (in blocks of NB sweeps) and
-//      the stage-1 panels (compact WY, GEMMs), applied to the eigenvectors.
+//   1. dense -> band of width NB (band_reduce.cu): per panel of NB columns a Householder QR, on one cluster of
+//      16 CTAs with the panel in shared memory and one cluster barrier per column (a cooperative kernel with a grid
+//      barrier where no such cluster can be placed), then the two-sided update of the trailing matrix as FP64
+//      tensor-core GEMMs; a panel is factorised on a second stream beside the update it does not need;
+//   2. band -> tridiagonal (bulge.cu): bulge chasing (sweeps of Householder reflectors of length NB, each annihilating
+//      one column and chasing the bulge down the band), a CTA per sweep, the sweeps taken by ticket from an ordinary
+//      launch;
+//   3. tridiagonal eigenpairs by divide and conquer, or the eigenvalues alone by bisection (tridiag_dc.cu);
+//   4. back-transformation: the stage-2 reflectors in blocks of NB sweeps (q2_apply.cu), then the stage-1 panels
+//      merged eight at a time (compact WY, GEMMs), their T factors made on the second stream beside step 2.
 #include <algorithm>
 #include <cmath>
 #include <vector>
-
-#include <cooperative_groups.h>
 
 #include "aux_join.h"
 #include "ctx.h"
@@ -56,14 +52,14 @@ __global__ void q1_gather_kernel(int m0, Q1Panels P, double *Vg)
     Vg[idx] = v;
 }
 
-// The same T from the panels' own T factors (T1) and the Gram blocks, merging pairs as
-// Q_a Q_b = I - [V_a V_b] [[T_a, -T_a G_ab T_b], [0, T_b]] [V_a V_b]^T (the block form of the
-// recurrence above): two 32 x 32 merges, then one of the 64-column halves; small products in
-// shared memory instead of 128 dependent column steps.
+// T of the merged reflector of four consecutive panels (q0 .. q0+3 of the group) from the panels' own T factors
+// (T1) and the Gram blocks G = V^T V, merging pairs as
+// Q_a Q_b = I - [V_a V_b] [[T_a, -T_a G_ab T_b], [0, T_b]] [V_a V_b]^T:
+// two 32 x 32 merges, then one of the 64-column halves; small products in shared memory instead of the 128 dependent
+// column steps of T(0:c, c) = -tau_c T(0:c, 0:c) G(0:c, c).  G and the output block T are Q1H x Q1H with leading
+// dimension Q1W.
 constexpr int Q1M_SMEM = (Q1H * (Q1H + 1) + 64 * 65) * (int)sizeof(double);
 
-// T of the merged reflector of four consecutive panels (q0 .. q0+3 of the group): G and the
-// output block T are Q1H x Q1H with leading dimension Q1W
 __global__ void __launch_bounds__(Q1H) q1_tmerge_kernel(const double *__restrict__ G, Q1Panels P, int q0,
                                                         const double *__restrict__ T1, int p0, double *Tg)
 {
@@ -104,12 +100,6 @@ __global__ void __launch_bounds__(Q1H) q1_tmerge_kernel(const double *__restrict
 
 }  // namespace
 
-}  // namespace bsrg
-
-namespace bsrg {
-
-
-// Workspace of dense_syevd in doubles (everything but the output Z)
 // ---------------------------------------------------------------------------
 // the working copy, its scale, and what a non-finite entry gives
 // ---------------------------------------------------------------------------
@@ -234,6 +224,7 @@ static Syevd2Layout syevd2_layout(int n, bool vectors)
     return L;
 }
 
+// workspace of dense_syevd in doubles (everything but the output Z)
 size_t syevd2_workspace_doubles(int n, bool vectors) { return syevd2_layout(n, vectors).total; }
 
 // the panels of group gq, their V in V1
@@ -307,8 +298,8 @@ static int syevd2_status(bsrg_ctx *c, const char *who, const int *flags, int *in
     return BSRG_OK;
 }
 
-// Eigenvalues (ascending, w) and eigenvectors (Z, ldz) of the symmetric A (lower
-// triangle referenced).  Z may be A itself.  ws: syevd2_workspace_doubles(n).
+// Eigenvalues (ascending, w) and eigenvectors (Z, ldz; null: none) of the symmetric A (lower
+// triangle referenced).  Z may be A itself.  ws: syevd2_workspace_doubles(n, Z != null).
 // tri_d / tri_e non-null: stop after the reduction and copy the tridiagonal (d: n, e: n-1) there
 static int syevd2_impl(bsrg_ctx *c, int n, const double *A, long lda, double *w, double *Z, long ldz, double *ws,
                        size_t ws_doubles, void *pinned, size_t pinned_bytes, int *launches, double *tri_d,

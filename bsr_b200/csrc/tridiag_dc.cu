@@ -12,20 +12,17 @@
 //     |b| at the cut);
 //   * leaves: one CTA each, cyclic Jacobi with tournament ordering on the dense
 //     leaf in shared memory;
-//   * merges, one tree level at a time, deepest first: per merge one CTA sorts
-//     the poles, finds the tolerance and runs the (sequential) deflation pass
-//     -- small z components and close poles merged by a Givens rotation --
-//     and lays the surviving columns out by type (upper half only, mixed, lower
-//     half only, deflated); the secular equation
-//     1 + rho sum z_i^2 / (d_i - lambda) = 0 is solved per root (bracketed
-//     Newton, every iterate kept inside a bisection bracket, roots stored as
-//     pole + offset); z is recomputed from the roots (Loewner's formula) and
-//     the eigenvectors of D + rho z z^T formed column by column; two FP64
-//     tensor-core GEMMs per merge (the rows of each half against its column
-//     types) give the merged eigenvectors, and a final pass writes eigenvalues
-//     and columns in ascending order.
-//   The per-level deflation counts are read back to the host once per level
-//   (they size the GEMMs).
+//   * merges, one tree level at a time, deepest first: per merge one CTA sorts the poles, finds the tolerance and
+//     deflates -- small z components, and close poles merged by a Givens rotation; every thread tests its pairs,
+//     only the rotations themselves are a chain -- and lays the surviving columns out by type (upper half only,
+//     mixed, lower half only, deflated); the secular equation 1 + rho sum z_i^2 / (d_i - lambda) = 0 is solved per
+//     root (two-pole rational iteration, every iterate kept inside a bracket, roots stored as pole + offset); z is
+//     recomputed from the roots (Loewner's formula) and the eigenvectors of D + rho z z^T formed column by column;
+//     all merged eigenvectors of a level, each half's rows against its column types, are one launch of FP64
+//     tensor-core products that writes the columns to their ascending places.
+//   The merges' sizes stay on the device (the launches cover the largest a merge can be), so nothing is read back
+//   between the levels.
+//   * eigenvalues alone: bisection on Sturm counts (tridiag_values).
 #include <algorithm>
 #include <cmath>
 #include <vector>
