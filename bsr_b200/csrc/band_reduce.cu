@@ -43,8 +43,7 @@ __device__ bool grid_sync(unsigned *bar, int *err, unsigned nblocks)
         }
         __threadfence();
     }
-    __syncthreads();
-    return *(volatile int *)err == 0;
+    return __syncthreads_or(*(volatile int *)err) == 0;      // the whole CTA goes on, or none of it
 }
 
 // ---------------------------------------------------------------------------

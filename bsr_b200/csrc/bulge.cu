@@ -407,8 +407,10 @@ __global__ void __launch_bounds__(BULGE_NT, 1) bulge_kernel(BulgeArgs a)
                 if (t == 0) *(volatile int *)&s.doneD = i + 1;
             }
         }
+        // (in this CTA's shared memory, so that its threads agree; a CTA that has not waited in vain finds the flag in
+        // its next wait)
         __syncthreads();
-        if (*(volatile int *)a.err) return;
+        if (*(volatile int *)&s.quit) return;
     }
 }
 

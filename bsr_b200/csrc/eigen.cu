@@ -85,8 +85,7 @@ __device__ __forceinline__ bool grid_barrier(const TrdArgs &a, unsigned gen)
             if (++it > TRD_SPIN_LIMIT) atomicExch(a.err, 1);
     }
     if (t == 0) __threadfence();
-    __syncthreads();
-    return *verr == 0;
+    return __syncthreads_or(*verr) == 0;                     // the whole CTA goes on, or none of it
 }
 
 // tiles per block edge for a trailing matrix of m rows: the largest that still
